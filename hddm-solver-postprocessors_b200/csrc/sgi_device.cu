@@ -450,16 +450,41 @@ __device__ __forceinline__ void load_row(const float* row, int o, bool in, float
 	else d[0] = in ? __ldg(row + o) : 0.f;
 }
 
-// QH: rows in flight per warp.  A window's hits are taken QH at a time in
-// index order: their rows are all loaded before the first is added, and the
-// adds follow the gold order.  Two rows suit large batches (registers buy
-// warps); small batches, whose few warps wait on each row, use more.
-template <int V, int E, int QH = 2>
-__global__ void __launch_bounds__(BLOCK) fwd_f64_kernel(const __grid_constant__ FwdArgs a)
+// A listed hit of the FP64 form.  Until its weight is known, `w` holds its
+// component range: {first component, component count} in two 32-bit words.
+struct __align__(16) Hit
 {
+	double w;
+	uint32_t node, pad;
+};
+
+// Hits a warp lists before it takes their weights and rows: a window adds at
+// most 32 to a list that holds fewer than 32.
+constexpr int HCAP = 64;
+
+__host__ __device__ __forceinline__ int hit_stride(int dim) { return 2 * HCAP + ((dim + 1) & ~1); }
+
+// FP64 form.  The walk only lists its hits (a window of 32 nodes holds two or
+// three of them); once 32 are listed, lane k takes hit k's weight, all lanes
+// busy, and the rows are then read QH at a time, QH such that a lane's loads
+// in flight fill 32 registers whatever the row width.  The adds follow the
+// list, which is in index order: gold's operations in gold's order.
+// Taking each window's hits at once instead (two rows in flight, the weights
+// of two or three busy lanes, then a wait for the rows) left the kernel
+// waiting on memory: 65,536 points on a regular 51,137-node grid of 32
+// outputs 14.6 ms against 8.9, ragged batches on six d=30 grids of 64
+// outputs 5.4 against 3.2, 131,072 points on a 150,000-node grid of 256
+// outputs 17.9 against 15.3 ms, where the L2 now runs at 80 % of its peak.
+template <int V, int E>
+__global__ void __launch_bounds__(BLOCK, 4) fwd_f64_kernel(const __grid_constant__ FwdArgs a)
+{
+	constexpr int QH = 16 / (V * E);
+	static_assert(32 % QH == 0, "groups of QH rows tile a full list");
 	extern __shared__ double smem[];
 	const int lane = threadIdx.x & 31;
-	double* xs = smem + (threadIdx.x >> 5) * a.dim;
+	double* wbase = smem + (threadIdx.x >> 5) * hit_stride(a.dim);
+	Hit* hits = reinterpret_cast<Hit*>(wbase);
+	double* xs = wbase + 2 * HCAP;
 	const bool first = a.chunk_begin == 0;
 	for (;;)
 	{
@@ -494,43 +519,84 @@ __global__ void __launch_bounds__(BLOCK) fwd_f64_kernel(const __grid_constant__ 
 			}
 		if (ok)
 		{
-			traverse<false>(G, xs, lane, lo, hi, [&](unsigned mask, int n0, double w, const uint4&, float)
+			const double* s64l = G.s64 + a.o_begin + out_col<E>(0, lane);
+			const uint32_t ld = (uint32_t)G.ld;
+			const int room = G.ld - a.o_begin - out_col<E>(0, lane);   // columns of a row from this lane's first
+			int n = 0;
+			// the first m <= 32 listed hits
+			auto take = [&](int m)
 			{
-				// QH hits per step, all their rows loaded before any is added, so
-				// that each warp keeps QH rows in flight; the adds stay in order
-				while (mask)
+				__syncwarp();
+				if (lane < m)
 				{
-					int kq[QH];
-#pragma unroll
-					for (int q = 0; q < QH; q++)
-					{
-						kq[q] = mask ? __ffs(mask) - 1 : -1;
-						if (mask) mask &= mask - 1;
-					}
+					const double t = hits[lane].w;
+					hits[lane].w = node_weight(G, xs, (uint32_t)__double2loint(t), (uint32_t)__double2hiint(t));
+				}
+				__syncwarp();
+				int h = 0;
+				for (; h + QH <= m; h += QH)
+				{
 					double sq[QH][V][E];
 #pragma unroll
 					for (int q = 0; q < QH; q++)
 					{
-						const double* row = G.s64 + (size_t)(n0 + (kq[q] >= 0 ? kq[q] : kq[0])) * G.ld + a.o_begin;
+						const double* row = s64l + (size_t)hits[h + q].node * ld;
 #pragma unroll
-						for (int v = 0; v < V; v++)
-						{
-							const int o = out_col<E>(v, lane);
-							load_row<E>(row, o, kq[q] >= 0 && a.o_begin + o < G.ld, sq[q][v]);
-						}
+						for (int v = 0; v < V; v++) load_row<E>(row, v * 32 * E, v * 32 * E < room, sq[q][v]);
 					}
 #pragma unroll
 					for (int q = 0; q < QH; q++)
 					{
-						if (kq[q] < 0) break;   // warp-uniform
-						const double wq = __shfl_sync(FULL, w, kq[q]);
+						const double wq = hits[h + q].w;
 #pragma unroll
 						for (int v = 0; v < V; v++)
 #pragma unroll
 							for (int e = 0; e < E; e++) acc[v][e] = __dadd_rn(acc[v][e], __dmul_rn(wq, sq[q][v][e]));
 					}
 				}
+				if (h < m)   // fewer than QH left (the point's last hits)
+				{
+					double sq[QH][V][E];
+#pragma unroll
+					for (int q = 0; q < QH; q++)
+					{
+						const double* row = s64l + (size_t)hits[min(h + q, m - 1)].node * ld;
+#pragma unroll
+						for (int v = 0; v < V; v++) load_row<E>(row, v * 32 * E, v * 32 * E < room && h + q < m, sq[q][v]);
+					}
+#pragma unroll
+					for (int q = 0; q < QH; q++)
+					{
+						if (h + q >= m) break;   // warp-uniform
+						const double wq = hits[h + q].w;
+#pragma unroll
+						for (int v = 0; v < V; v++)
+#pragma unroll
+							for (int e = 0; e < E; e++) acc[v][e] = __dadd_rn(acc[v][e], __dmul_rn(wq, sq[q][v][e]));
+					}
+				}
+			};
+			traverse<false>(G, xs, lane, lo, hi, [&](unsigned mask, int n0, double, const uint4& r, float)
+			{
+				if ((mask >> lane) & 1u)
+				{
+					Hit t;
+					t.w = __hiloint2double((int)(r.z & 0xffu), (int)r.y);
+					t.node = (uint32_t)(n0 + lane);
+					t.pad = 0u;
+					hits[n + __popc(mask & ((1u << lane) - 1u))] = t;
+				}
+				n += __popc(mask);
+				if (n >= 32)
+				{
+					take(32);
+					n -= 32;
+					__syncwarp();
+					if (lane < n) hits[lane] = hits[32 + lane];
+					__syncwarp();
+				}
 			}, nullptr, pathmask, a.chain_len[gi]);
+			if (n) take(n);
 		}
 #pragma unroll
 		for (int v = 0; v < V; v++)
@@ -1877,27 +1943,25 @@ void (*fp32c_kernel(int variant, bool descent, int cols))(FwdArgs)
 	return cols == V * 32 * E ? f32d_variant<V, E, true>(variant) : f32d_variant<V, E, false>(variant);
 }
 
-// small: a batch of fewer points than resident warps; the FP64 form then
-// keeps eight rows in flight per warp (four for eight outputs per lane).
-void (*select_fwd(int precision, int ld, int cols, int variant = 0, bool descent = false, bool small = false))(FwdArgs)
+void (*select_fwd(int precision, int ld, int cols, int variant = 0, bool descent = false))(FwdArgs)
 {
 	const bool f64 = precision == SGI_FP64;
-	if (ld <= 32) return f64 ? (small ? fwd_f64_kernel<1, 1, 8> : fwd_f64_kernel<1, 1>) : fp32c_kernel<1, 1>(variant, descent, cols);
-	if (cols <= 64) return f64 ? (small ? fwd_f64_kernel<1, 2, 8> : fwd_f64_kernel<1, 2>) : fp32c_kernel<1, 2>(variant, descent, cols);
+	if (ld <= 32) return f64 ? fwd_f64_kernel<1, 1> : fp32c_kernel<1, 1>(variant, descent, cols);
+	if (cols <= 64) return f64 ? fwd_f64_kernel<1, 2> : fp32c_kernel<1, 2>(variant, descent, cols);
 	// FP32C reads four consecutive outputs per lane (16-byte loads) when rows
 	// are a multiple of 128 wide
 	const bool e4 = !f64 && ld % 128 == 0;
 	if (cols <= 128)
-		return f64 ? (small ? fwd_f64_kernel<2, 2, 8> : fwd_f64_kernel<2, 2>)
+		return f64 ? fwd_f64_kernel<2, 2>
 		           : e4 ? fp32c_kernel<1, 4>(variant, descent, cols) : fp32c_kernel<2, 2>(variant, descent, cols);
-	return f64 ? (small ? fwd_f64_kernel<4, 2, 4> : fwd_f64_kernel<4, 2>)
+	return f64 ? fwd_f64_kernel<4, 2>
 	           : e4 ? fp32c_kernel<2, 4>(variant, descent, cols) : fp32c_kernel<4, 2>(variant, descent, cols);
 }
 
 // Dynamic shared memory of a forward launch.
 size_t fwd_smem(int precision, int dim, bool descent = false)
 {
-	if (precision != SGI_FP32C) return (size_t)WARPS * dim * sizeof(double);
+	if (precision != SGI_FP32C) return (size_t)WARPS * hit_stride(dim) * sizeof(double);
 	return (size_t)WARPS * (descent ? desc_stride(dim) : list_stride(dim)) * sizeof(double);
 }
 
@@ -2832,7 +2896,7 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 			CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream));
 			const int cols = std::min(g0->TD - ob, PASS);
 			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel
-				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, W->sms), descent, small);
+				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, W->sms), descent);
 			if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 			int blocks = 0;
 			rc = occupancy_grid(kern, smem, W->sms, &blocks);
@@ -3250,7 +3314,7 @@ extern "C" int sgi_interpolate_noalloc(int ngrids, const sgi_grid_t* grids, cons
 			CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream));
 			const int cols = std::min(g0->TD - ob, PASS);
 			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel
-				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, sms), descent, small);
+				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, sms), descent);
 			if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 			int blocks = 0;
 			rc = occupancy_grid(kern, smem, sms, &blocks);
