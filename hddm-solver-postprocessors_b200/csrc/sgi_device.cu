@@ -46,6 +46,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "sgi_internal.h"
@@ -1537,9 +1538,11 @@ __global__ void __launch_bounds__(LBLOCK) fwd_f64_list_kernel(const __grid_const
 // classes: classes[4p] big (FP64 row), [4p + 1] fine (FP32 row), [4p + 2]
 // fine (FP16 row), [4p + 3] dropped, by the bound |w| * max|s_row| of the
 // full-product weight.
+// `any`: points with a non-finite coordinate are walked too (their hats in
+// that dimension are not positive), as the backward walks them.
 template <bool CLASSES>
 __global__ void __launch_bounds__(BLOCK) count_kernel(const __grid_constant__ FwdArgs a, long long* counts,
-	long long* classes)
+	long long* classes, bool any)
 {
 	extern __shared__ double smem[];
 	const int lane = threadIdx.x & 31;
@@ -1552,7 +1555,7 @@ __global__ void __launch_bounds__(BLOCK) count_kernel(const __grid_constant__ Fw
 		if (p >= a.npts) break;
 		const GridDesc& G = a.g[find_grid(a, p)];
 		long long cnt = 0, nbig = 0, nfine = 0, nhalf = 0;
-		if (load_point(a, p, xs, lane))
+		if (load_point(a, p, xs, lane) || any)
 			traverse(G, xs, lane, [&](unsigned mask, int, double w, const uint4& r, float rm)
 			{
 				cnt += __popc(mask);
@@ -1585,19 +1588,34 @@ __global__ void __launch_bounds__(BLOCK) count_kernel(const __grid_constant__ Fw
 
 // ------------------------------------------------------------------ backward
 //
-// dL/dx: per point (one warp), for every active node n the scalar
-// cs = sum_o gout[p,o] * s[n,o] (warp reduction), then for each component c of
-// n, dw/dx_{dim c} = (prod of the other hats) * slope_c, slope = -i sign(x i - j).
-// dL/dsurplus: pairs (node, point, weight) are written at per-point offsets
-// (exclusive scan of the active counts: no atomics), stably radix-sorted by
-// node, and each node's segment is reduced by one warp in point order.
+// With w_np the weight of node n at point p and cs_np = sum_o gout[p,o] * s[n,o]:
+//   dL/dsurplus[n,:] = sum_p w_np * gout[p,:]
+//   dL/dx[p,d]       = sum_n cs_np * dw_np/dx_d,  dw/dx_d = w * slope_d / hat_d,
+//                      slope_d = -i sign(x_d i - j)
+// over the pairs (n, p) of active nodes.
+//
+// Both gradients (bwd_list_kernel, bwd_nodes_kernel, bwd_dx_kernel): the walk
+// writes every point's pairs at its offset (exclusive scan of the active
+// counts, no atomics); pair numbers are stably radix-sorted by node; each
+// pair's gout row is then read once, for its node's dL/dsurplus sum and for
+// the pair's cs (the node's surplus row stays in registers); cs * w replaces w
+// in the pair; one warp per point adds its pairs' dL/dx.  The row gathers are
+// what bounds it, and of the two sides gout is the smaller one (33 MB against
+// 300 MB of surplus rows for 32,768 points of a 300,000-node grid of 128
+// outputs), so its rows come from the L2.  That case: 17.9 ms with surplus
+// rows gathered per point for cs (13.4 ms of it) and gout rows per node, one
+// warp per node, for the sums (6.2); now 6.4 ms, of which the rows take 2.5
+// (14 TB/s, L1 at 77 % of its peak), dL/dx 2, the sort 1.1, the two walks 1.5.
+// dL/dx alone (bwd_points_kernel): the pairs stay with their point, which
+// gathers the surplus rows of 32 hits at a time (5,001 points, 50,000 nodes,
+// 118 outputs: 1.60 ms with two rows at a time, now 0.64).
 
-// One (point, weight) pair of the dL/dsurplus reduction, sorted by node with
-// its node as the key.
-struct PairVal
+// One pair of the dL/dsurplus reduction, in point order: the weight, then
+// cs * w once the node's warp has it.
+struct __align__(16) PairVal
 {
-	uint32_t point, pad;
 	double w;
+	uint32_t point, pad;
 };
 
 struct BwdArgs
@@ -1606,20 +1624,236 @@ struct BwdArgs
 	const double* x;
 	const double* gout;
 	double* gx;
-	const long long* pair_off;   // npts + 1, or null
-	uint32_t* pair_node;
+	double* gs;
+	const long long* pair_off;   // npts + 1
+	uint32_t* pair_node;         // per pair, in point order: node, its value, its number
 	PairVal* pair_val;
+	uint32_t* pair_idx;
+	const uint32_t* sorted_node; // sorted by node: node, pair number
+	const uint32_t* sorted_idx;
+	double* part;                // sums of nodes cut by tile ends, 2 per tile of PART pairs
 	unsigned long long* counter;
-	long long npts;
+	long long npts, npairs;
 	int dim, TD;
 };
 
+// Sums of C values per lane over the warp: lane l gets value l >> (5 - log2 C).
+// Halving exchanges: C - 1 of them, then log2(32 / C) butterflies, against 5 C
+// for one butterfly per value.
+template <int C>
+__device__ __forceinline__ double warp_sums(double* c, int lane)
+{
+	int bit = 16;
+#pragma unroll
+	for (int n = C; n > 1; n >>= 1, bit >>= 1)
+#pragma unroll
+		for (int j = 0; j < n / 2; j++)
+		{
+			const bool up = lane & bit;
+			const double keep = up ? c[j + n / 2] : c[j];
+			const double send = up ? c[j] : c[j + n / 2];
+			c[j] = keep + __shfl_xor_sync(FULL, send, bit);
+		}
+	double t = c[0];
+#pragma unroll
+	for (; bit > 0; bit >>= 1) t += __shfl_xor_sync(FULL, t, bit);
+	return t;
+}
+
+// Rows of R outputs per lane that go through registers together (32 registers
+// of loads in flight); their products are summed over the warp CB at a time.
+template <int R> struct RowGroup
+{
+	static constexpr int QB = R >= 8 ? 2 : R == 4 ? 4 : 8;
+	static constexpr int CB = 8;
+};
+
+// Column of a lane's r-th output of R: one column per lane up to 32, else two
+// neighbours per 64 columns, so that a row is read 16 bytes per lane.
 template <int R>
-__global__ void __launch_bounds__(BLOCK) bwd_points_kernel(const __grid_constant__ BwdArgs a)
+__device__ __forceinline__ int bwd_col(int r, int lane) { return R == 1 ? lane : 64 * (r >> 1) + 2 * lane + (r & 1); }
+
+// A lane's outputs of a row of `cols` columns, zero past them.  VEC: `cols` is
+// even and the row starts on a 16-byte boundary.
+template <int R, bool VEC>
+__device__ __forceinline__ void bwd_row(const double* row, int cols, int lane, double* v)
+{
+	if constexpr (R == 1) v[0] = lane < cols ? __ldg(row + lane) : 0.0;
+	else
+#pragma unroll
+		for (int r = 0; r < R; r += 2)
+		{
+			const int o = bwd_col<R>(r, lane);
+			if constexpr (VEC)
+			{
+				const double2 t = o < cols ? __ldg(reinterpret_cast<const double2*>(row + o)) : make_double2(0.0, 0.0);
+				v[r] = t.x;
+				v[r + 1] = t.y;
+			}
+			else
+			{
+				v[r] = o < cols ? __ldg(row + o) : 0.0;
+				v[r + 1] = o + 1 < cols ? __ldg(row + o + 1) : 0.0;
+			}
+		}
+}
+
+// The products of the m <= 32 surplus rows base + ld * row_k (lane k holds
+// row_k) with `mul`, to lane k.
+template <int R>
+__device__ __forceinline__ double rows_dot(const double* base, uint32_t ld, uint32_t row, int m, int lane, const double* mul)
+{
+	constexpr int QB = RowGroup<R>::QB, CB = RowGroup<R>::CB;
+	double dot = 0.0;
+	for (int k = 0; k < m; k += CB)
+	{
+		double c[CB];
+#pragma unroll
+		for (int h = 0; h < CB; h += QB)
+		{
+			double v[QB][R];
+#pragma unroll
+			for (int q = 0; q < QB; q++)
+			{
+				const uint32_t n = __shfl_sync(FULL, row, min(k + h + q, m - 1));
+				bwd_row<R, true>(base + (size_t)n * ld, k + h + q < m ? (int)ld : 0, lane, v[q]);
+			}
+#pragma unroll
+			for (int q = 0; q < QB; q++)
+			{
+				c[h + q] = 0.0;
+#pragma unroll
+				for (int r = 0; r < R; r++) c[h + q] = fma(mul[r], v[q][r], c[h + q]);
+			}
+		}
+		const double u = __shfl_sync(FULL, warp_sums<CB>(c, lane), (lane & (CB - 1)) << 2);
+		if (lane - k >= 0 && lane - k < CB) dot = u;
+	}
+	return dot;
+}
+
+// 1/h for h in [2^-53, 1]: two Newton-Raphson steps from the approximate
+// reciprocal, within an ulp or two.
+__device__ __forceinline__ double rcp_hat(double h)
+{
+	double r;
+	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(h));
+	r = fma(r, fma(-h, r, 1.0), r);
+	return fma(r, fma(-h, r, 1.0), r);
+}
+
+// dL/dx terms of m <= 32 pairs of one point (lane k holds pair k's component
+// range and cs * w): each half-warp takes every other pair, a component per
+// lane (a node of a d=59 grid has ten on average), and adds to its own copy of
+// the point's gradient (gxs, gxs + dim), so that two pairs sharing a dimension
+// never meet.  dw/dx as w * slope / hat needs no products of the other hats;
+// eight pairs' components are in flight while eight are added (with two, the
+// loads were what it waited on: 2.6 ms against 2.2 over 44M pairs).
+__device__ __forceinline__ void dx_pass(const GridDesc& G, const double* xs, double* gxs, int dim, uint32_t cptr,
+	uint32_t ncomp, double csw, int m, int lane)
+{
+	constexpr int U = 4;   // pairs a half-warp has in flight
+	const int half = lane >> 4, l = lane & 15;
+	double* gh = gxs + half * dim;
+	uint2 nx[U];
+	auto fetch = [&](int k)
+	{
+#pragma unroll
+		for (int u = 0; u < U; u++)
+		{
+			const int q = k + 2 * u + half;
+			const uint32_t cp = __shfl_sync(FULL, cptr, min(q, 31)), nc = __shfl_sync(FULL, ncomp, min(q, 31));
+			nx[u] = q < m && (uint32_t)l < nc ? __ldg(G.comps + cp + l) : make_uint2(0u, 0u);
+		}
+	};
+	fetch(0);
+	for (int k = 0; k < m; k += 2 * U)
+	{
+		uint2 c[U];
+#pragma unroll
+		for (int u = 0; u < U; u++) c[u] = nx[u];
+		if (k + 2 * U < m) fetch(k + 2 * U);
+#pragma unroll
+		for (int u = 0; u < U; u++)
+		{
+			const int p = k + 2 * u + half;
+			const double a = __shfl_sync(FULL, csw, min(p, 31));
+			const uint32_t n = __shfl_sync(FULL, ncomp, min(p, 31)), nc = p < m ? n : 0u;
+			const uint32_t cp = __shfl_sync(FULL, cptr, min(p, 31));
+			uint32_t q = l;
+			do
+			{
+				if (q < nc)
+				{
+					const uint2 cc = q < 16u ? c[u] : __ldg(G.comps + cp + q);
+					const double xd = xs[cc.x];
+					const double i = u32_to_double(cc.y & 0xffffu), j = u32_to_double(cc.y >> 16);
+					// slope -i sign(x i - j): i's sign bit from the difference
+					const double t = fma(xd, i, -j);
+					const double slope = __hiloint2double(__double2hiint(i) | (~__double2hiint(t) & 0x80000000), __double2loint(i));
+					const double h = __dsub_rn(1.0, fabs(__dsub_rn(__dmul_rn(xd, i), j)));   // as hat()
+					const double v = a * slope * rcp_hat(h);
+					if (t != 0.0) gh[cc.x] += v;
+				}
+				__syncwarp();
+				q += 16;
+			} while (__any_sync(FULL, q < nc));
+		}
+	}
+}
+
+__host__ __device__ __forceinline__ int bwd_stride(int dim) { return HCAP * 2 + 3 * dim + (dim & 1); }
+
+// Walks point p's active nodes and hands them over in lists of at most 32 in
+// index order: on_list(m, hit) with lane k < m holding hit k (its component
+// range in w, see Hit).
+template <class OnList>
+__device__ __forceinline__ void walk_lists(const GridDesc& G, const double* xs, Hit* hits, int lane, OnList&& on_list)
+{
+	int n = 0;
+	auto take = [&](int m)
+	{
+		__syncwarp();
+		Hit h;
+		h.w = 0.0; h.node = 0u; h.pad = 0u;
+		if (lane < m) h = hits[lane];
+		on_list(m, h);
+	};
+	traverse<false>(G, xs, lane, 0, G.nno, [&](unsigned mask, int n0, double, const uint4& r, float)
+	{
+		if ((mask >> lane) & 1u)
+		{
+			Hit t;
+			t.w = __hiloint2double((int)(r.z & 0xffu), (int)r.y);
+			t.node = (uint32_t)(n0 + lane);
+			t.pad = 0u;
+			hits[n + __popc(mask & ((1u << lane) - 1u))] = t;
+		}
+		n += __popc(mask);
+		if (n >= 32)
+		{
+			take(32);
+			n -= 32;
+			__syncwarp();
+			if (lane < n) hits[lane] = hits[32 + lane];
+			__syncwarp();
+		}
+	});
+	if (n) take(n);
+}
+
+__device__ __forceinline__ uint32_t hit_cptr(const Hit& h) { return (uint32_t)__double2loint(h.w); }
+__device__ __forceinline__ uint32_t hit_ncomp(const Hit& h) { return (uint32_t)__double2hiint(h.w); }
+
+// dL/dx without dL/dsurplus: one warp per point, 32 hits at a time.
+template <int R>
+__global__ void __launch_bounds__(BLOCK, R == 8 ? 2 : 3) bwd_points_kernel(const __grid_constant__ BwdArgs a)
 {
 	extern __shared__ double smem[];
 	const int lane = threadIdx.x & 31;
-	double* xs = smem + (threadIdx.x >> 5) * 2 * a.dim;
+	double* wbase = smem + (threadIdx.x >> 5) * bwd_stride(a.dim);
+	Hit* hits = reinterpret_cast<Hit*>(wbase);
+	double* xs = wbase + 2 * HCAP;
 	double* gxs = xs + a.dim;
 	const GridDesc& G = a.G;
 	for (;;)
@@ -1628,174 +1862,266 @@ __global__ void __launch_bounds__(BLOCK) bwd_points_kernel(const __grid_constant
 		if (lane == 0) p = (long long)atomicAdd(a.counter, 1ull);
 		p = __shfl_sync(FULL, p, 0);
 		if (p >= a.npts) break;
-		for (int k = lane; k < a.dim; k += 32) { xs[k] = a.x[(size_t)p * a.dim + k]; gxs[k] = 0.0; }
+		for (int k = lane; k < a.dim; k += 32) { xs[k] = a.x[(size_t)p * a.dim + k]; gxs[k] = 0.0; gxs[a.dim + k] = 0.0; }
 		double g[R];
-#pragma unroll
-		for (int r = 0; r < R; r++)
-		{
-			const int o = lane + 32 * r;
-			g[r] = o < a.TD ? a.gout[(size_t)p * a.TD + o] : 0.0;
-		}
+		bwd_row<R, false>(a.gout + (size_t)p * a.TD, a.TD, lane, g);
 		__syncwarp();
-		long long woff = a.pair_off ? a.pair_off[p] : 0;
-		traverse(G, xs, lane, [&](unsigned mask, int n0, double w, const uint4& rec, float)
+		walk_lists(G, xs, hits, lane, [&](int m, const Hit& h)
 		{
-			if (a.pair_off)
-			{
-				const int rank = __popc(mask & ((1u << lane) - 1u));
-				if ((mask >> lane) & 1u)
-				{
-					a.pair_node[woff + rank] = (uint32_t)(n0 + lane);
-					a.pair_val[woff + rank] = PairVal{ (uint32_t)p, 0u, w };
-				}
-				woff += __popc(mask);
-			}
-			if (!a.gx) return;
-			// dx contribution of hit k with cs = sum_o gout[o] * s[node, o]
-			auto components = [&](int k, double cs)
-			{
-				const uint32_t cptr = __shfl_sync(FULL, rec.y, k);
-				const uint32_t ncomp = __shfl_sync(FULL, rec.z, k) & 0xffu;
-				if (ncomp <= 32)
-				{
-					// lane c holds component c's hat and slope; the product of the
-					// other hats is the exclusive prefix times the exclusive suffix
-					// product over the lanes (lanes past ncomp hold 1)
-					double h = 1.0, slope = 0.0;
-					uint32_t dc = 0;
-					if ((uint32_t)lane < ncomp)
-					{
-						const uint2 cp = __ldg(G.comps + cptr + lane);
-						dc = cp.x;
-						h = hat(xs[cp.x], cp.y);
-						const double t = xs[cp.x] * (double)(cp.y & 0xffffu) - (double)(cp.y >> 16);
-						slope = t > 0.0 ? -(double)(cp.y & 0xffffu) : (t < 0.0 ? (double)(cp.y & 0xffffu) : 0.0);
-					}
-					double pre = h, suf = h;
-	#pragma unroll
-					for (int off = 1; off < 32; off <<= 1)
-					{
-						const double u = __shfl_up_sync(FULL, pre, off);
-						const double d = __shfl_down_sync(FULL, suf, off);
-						if (lane >= off) pre *= u;
-						if (lane + off < 32) suf *= d;
-					}
-					double before = __shfl_up_sync(FULL, pre, 1), after = __shfl_down_sync(FULL, suf, 1);
-					if (lane == 0) before = 1.0;
-					if (lane == 31) after = 1.0;
-					if ((uint32_t)lane < ncomp) gxs[dc] += cs * (before * after) * slope;
-				}
-				else
-					for (uint32_t c = lane; c < ncomp; c += 32)
-					{
-						const uint2 cp = __ldg(G.comps + cptr + c);
-						double others = 1.0;
-						for (uint32_t q = 0; q < ncomp; q++)
-							if (q != c)
-							{
-								const uint2 cq = __ldg(G.comps + cptr + q);
-								others *= hat(xs[cq.x], cq.y);
-							}
-						const double t = xs[cp.x] * (double)(cp.y & 0xffffu) - (double)(cp.y >> 16);
-						const double slope = t > 0.0 ? -(double)(cp.y & 0xffffu) : (t < 0.0 ? (double)(cp.y & 0xffffu) : 0.0);
-						gxs[cp.x] += cs * others * slope;
-					}
-				__syncwarp();
-			};
-			// two hits at a time: both rows loaded and reduced together; their
-			// dx contributions are added one after the other (they may share
-			// dimensions)
-			while (mask)
-			{
-				const int k0 = __ffs(mask) - 1;
-				mask &= mask - 1;
-				const bool two = mask != 0u;
-				const int k1 = two ? __ffs(mask) - 1 : k0;
-				if (two) mask &= mask - 1;
-				const double* row0 = G.s64 + (size_t)(n0 + k0) * G.ld;
-				const double* row1 = G.s64 + (size_t)(n0 + k1) * G.ld;
-				double s0[R], s1[R];
-#pragma unroll
-				for (int r = 0; r < R; r++)
-				{
-					const int o = lane + 32 * r;
-					s0[r] = o < a.TD ? __ldg(row0 + o) : 0.0;
-					s1[r] = (two && o < a.TD) ? __ldg(row1 + o) : 0.0;
-				}
-				double cs0 = 0.0, cs1 = 0.0;
-#pragma unroll
-				for (int r = 0; r < R; r++) { cs0 = fma(g[r], s0[r], cs0); cs1 = fma(g[r], s1[r], cs1); }
-#pragma unroll
-				for (int off = 16; off > 0; off >>= 1)
-				{
-					cs0 += __shfl_xor_sync(FULL, cs0, off);
-					cs1 += __shfl_xor_sync(FULL, cs1, off);
-				}
-				components(k0, cs0);
-				if (two) components(k1, cs1);
-			}
+			const double w = lane < m ? node_weight(G, xs, hit_cptr(h), hit_ncomp(h)) : 0.0;
+			const double cs = rows_dot<R>(G.s64, (uint32_t)G.ld, h.node, m, lane, g);
+			dx_pass(G, xs, gxs, a.dim, hit_cptr(h), hit_ncomp(h), cs * w, m, lane);
 		});
-		if (a.gx)
-			for (int k = lane; k < a.dim; k += 32) a.gx[(size_t)p * a.dim + k] = gxs[k];
+		__syncwarp();
+		for (int k = lane; k < a.dim; k += 32) a.gx[(size_t)p * a.dim + k] = gxs[k] + gxs[a.dim + k];
 		__syncwarp();
 	}
 }
 
-// One warp per node: dL/dsurplus[n, :] = sum over its pairs of w * gout[point, :],
-// in sorted (point) order.  The node's pairs are read 32 at a time (lane l
-// loads pair q + l) and their gout rows two at a time.
-template <int R>
-__global__ void __launch_bounds__(BLOCK) bwd_surplus_kernel(const uint32_t* __restrict__ sorted_node,
-	const PairVal* __restrict__ sorted_val, long long npairs, const double* __restrict__ gout,
-	double* __restrict__ gs, int nno, int TD)
+// Every point's pairs, in index order, at its offset.
+__global__ void __launch_bounds__(BLOCK) bwd_list_kernel(const __grid_constant__ BwdArgs a)
 {
+	extern __shared__ double smem[];
 	const int lane = threadIdx.x & 31;
-	const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-	for (long long n = warp; n < nno; n += nwarps)
+	double* wbase = smem + (threadIdx.x >> 5) * hit_stride(a.dim);
+	Hit* hits = reinterpret_cast<Hit*>(wbase);
+	double* xs = wbase + 2 * HCAP;
+	const GridDesc& G = a.G;
+	for (;;)
 	{
-		// segment [lo, e) of node n in the sorted keys
-		long long lo = 0, hi = npairs;
-		while (lo < hi) { long long m = (lo + hi) >> 1; if (sorted_node[m] < (uint32_t)n) lo = m + 1; else hi = m; }
-		long long e = lo, h2 = npairs;
-		while (e < h2) { long long m = (e + h2) >> 1; if (sorted_node[m] <= (uint32_t)n) e = m + 1; else h2 = m; }
-		double acc[R];
-#pragma unroll
-		for (int r = 0; r < R; r++) acc[r] = 0.0;
-		for (long long q0 = lo; q0 < e; q0 += 32)
+		long long p = 0;
+		if (lane == 0) p = (long long)atomicAdd(a.counter, 1ull);
+		p = __shfl_sync(FULL, p, 0);
+		if (p >= a.npts) break;
+		for (int k = lane; k < a.dim; k += 32) xs[k] = a.x[(size_t)p * a.dim + k];
+		__syncwarp();
+		long long at = a.pair_off[p];
+		walk_lists(G, xs, hits, lane, [&](int m, const Hit& h)
 		{
-			const int m = (int)min(32ll, e - q0);
-			PairVal pv{ 0u, 0u, 0.0 };
-			if (lane < m) pv = sorted_val[q0 + lane];
-			for (int k = 0; k < m; k += 2)
+			if (lane < m)
 			{
-				const bool two = k + 1 < m;
-				const double w0 = __shfl_sync(FULL, pv.w, k);
-				const double w1 = __shfl_sync(FULL, pv.w, two ? k + 1 : k);
-				const double* r0 = gout + (size_t)__shfl_sync(FULL, pv.point, k) * TD;
-				const double* r1 = gout + (size_t)__shfl_sync(FULL, pv.point, two ? k + 1 : k) * TD;
-				double v0[R], v1[R];
+				a.pair_node[at + lane] = h.node;
+				a.pair_val[at + lane] = PairVal{ node_weight(G, xs, hit_cptr(h), hit_ncomp(h)), (uint32_t)p, 0u };
+				a.pair_idx[at + lane] = (uint32_t)(at + lane);
+			}
+			at += m;
+		});
+		__syncwarp();
+	}
+}
+
+// dL/dsurplus and the pairs' cs * w: the sorted pairs are cut into tiles of
+// PART, one warp each, so that a node of many pairs (the root is active for
+// every point) is spread over warps and one of few costs no start-up: the rows
+// stream through, QB at a time, across node boundaries.  A node's sum goes to
+// gs when the tile holds all its pairs, else to `part`: the tile's first node
+// when it began before the tile to sum 2 t, a node that goes on after it to
+// sum 2 t + 1 (2 t when it covers the tile's first pair); bwd_join_kernel adds
+// them in order.  Pair numbers are loaded two batches of 32 ahead, the pairs
+// they name one ahead.
+constexpr long long PART = 1024;
+
+template <int R, bool DOT, bool VEC>
+__global__ void __launch_bounds__(BLOCK, R == 8 ? 2 : 3) bwd_nodes_kernel(const __grid_constant__ BwdArgs a)
+{
+	constexpr int QB = RowGroup<R>::QB, CB = RowGroup<R>::CB;
+	__shared__ PairVal batch[WARPS][32];   // this batch's pairs: one 16-byte read per row instead of three shuffles
+	const int lane = threadIdx.x & 31;
+	PairVal* pairs = batch[threadIdx.x >> 5];
+	const GridDesc& G = a.G;
+	const int TD = a.TD;
+	const uint32_t ld = (uint32_t)a.TD;
+	const long long ntiles = (a.npairs + PART - 1) / PART;
+	for (;;)
+	{
+		long long it = 0;
+		if (lane == 0) it = (long long)atomicAdd(a.counter, 1ull);
+		it = __shfl_sync(FULL, it, 0);
+		if (it >= ntiles) break;
+		const long long tb = it * PART, te = min(tb + PART, a.npairs);
+		uint32_t cur = __ldg(a.sorted_node + tb);
+		bool carried = tb > 0 && __ldg(a.sorted_node + tb - 1) == cur;   // began before the tile
+		const bool goes_on = te < a.npairs && __ldg(a.sorted_node + te) == __ldg(a.sorted_node + te - 1);
+		bool at_start = true;                                            // `cur` covers the tile's first pair
+		double mul[R], acc[R];
+		auto begin = [&](uint32_t n)
+		{
+			cur = n;
+			if (DOT) bwd_row<R, true>(G.s64 + (size_t)n * G.ld, G.ld, lane, mul);
 #pragma unroll
-				for (int r = 0; r < R; r++)
+			for (int r = 0; r < R; r++) acc[r] = 0.0;
+		};
+		auto store = [&](double* dst)
+		{
+#pragma unroll
+			for (int r = 0; r < R; r++)
+			{
+				const int o = bwd_col<R>(r, lane);
+				if (o < TD) dst[o] = acc[r];
+			}
+		};
+		begin(cur);
+		uint32_t node1 = 0u, idx1 = 0u, node2 = 0u, idx2 = 0u;   // this batch's, the next one's
+		PairVal pv1{ 0.0, 0u, 0u };
+		if (tb + lane < te)
+		{
+			node1 = __ldg(a.sorted_node + tb + lane);
+			idx1 = __ldg(a.sorted_idx + tb + lane);
+			pv1 = a.pair_val[idx1];
+		}
+		if (tb + 32 + lane < te)
+		{
+			node2 = __ldg(a.sorted_node + tb + 32 + lane);
+			idx2 = __ldg(a.sorted_idx + tb + 32 + lane);
+		}
+		for (long long b = tb; b < te; b += 32)
+		{
+			const int m = (int)min(32ll, te - b);
+			const uint32_t node = node1, idx = idx1;
+			const PairVal pv = pv1;
+			node1 = node2; idx1 = idx2;
+			if (b + 32 + lane < te) pv1 = a.pair_val[idx2];
+			if (b + 64 + lane < te)
+			{
+				node2 = __ldg(a.sorted_node + b + 64 + lane);
+				idx2 = __ldg(a.sorted_idx + b + 64 + lane);
+			}
+			const uint32_t before = __shfl_up_sync(FULL, node, 1);
+			const unsigned bounds = __ballot_sync(FULL, lane < m && node != (lane ? before : cur));
+			__syncwarp();
+			pairs[lane] = pv;
+			__syncwarp();
+			double dot = 0.0;
+			for (int k = 0; k < m; k += CB)
+			{
+				if (k + CB <= m && !((bounds >> k) & ((1u << CB) - 1u)))
 				{
-					const int o = lane + 32 * r;
-					v0[r] = o < TD ? r0[o] : 0.0;
-					v1[r] = (two && o < TD) ? r1[o] : 0.0;
+					double c[CB];
+#pragma unroll
+					for (int h = 0; h < CB; h += QB)
+					{
+						double v[QB][R], wq[QB];
+#pragma unroll
+						for (int q = 0; q < QB; q++)
+						{
+							const PairVal pq = pairs[k + h + q];
+							wq[q] = pq.w;
+							bwd_row<R, VEC>(a.gout + (size_t)pq.point * ld, TD, lane, v[q]);
+						}
+#pragma unroll
+						for (int q = 0; q < QB; q++)
+						{
+							c[h + q] = 0.0;
+#pragma unroll
+							for (int r = 0; r < R; r++)
+							{
+								acc[r] = fma(wq[q], v[q][r], acc[r]);
+								if (DOT) c[h + q] = fma(mul[r], v[q][r], c[h + q]);
+							}
+						}
+					}
+					if (DOT)
+					{
+						const double u = __shfl_sync(FULL, warp_sums<CB>(c, lane), (lane & (CB - 1)) << 2);
+						if (lane - k >= 0 && lane - k < CB) dot = u;
+					}
+					continue;
 				}
-#pragma unroll
-				for (int r = 0; r < R; r++)
+				// a node begins among these rows, or fewer than CB are left: one at a time
+				for (int q = k; q < min(k + CB, m); q++)
 				{
-					acc[r] = fma(w0, v0[r], acc[r]);
-					if (two) acc[r] = fma(w1, v1[r], acc[r]);
+					if ((bounds >> q) & 1u)
+					{
+						store(at_start && carried ? a.part + (size_t)(2 * it) * TD : a.gs + (size_t)cur * TD);
+						at_start = false;
+						begin(__shfl_sync(FULL, node, q));
+					}
+					const double wq = pairs[q].w;
+					double v[R], c[1] = { 0.0 };
+					bwd_row<R, VEC>(a.gout + (size_t)pairs[q].point * ld, TD, lane, v);
+#pragma unroll
+					for (int r = 0; r < R; r++)
+					{
+						acc[r] = fma(wq, v[r], acc[r]);
+						if (DOT) c[0] = fma(mul[r], v[r], c[0]);
+					}
+					if (DOT)
+					{
+						const double t = warp_sums<1>(c, lane);   // every lane has the sum
+						if (lane == q) dot = t;
+					}
 				}
 			}
+			if (DOT && lane < m) a.pair_val[idx].w = dot * pv.w;
 		}
-#pragma unroll
-		for (int r = 0; r < R; r++)
+		if (goes_on) store(a.part + (size_t)(2 * it + (at_start ? 0 : 1)) * TD);
+		else store(at_start && carried ? a.part + (size_t)(2 * it) * TD : a.gs + (size_t)cur * TD);
+	}
+}
+
+// Nodes cut by tile ends: their parts' sums, added in order, by the warp of
+// the tile in which the node begins.
+__global__ void __launch_bounds__(BLOCK) bwd_join_kernel(const __grid_constant__ BwdArgs a)
+{
+	const int lane = threadIdx.x & 31;
+	const uint32_t* key = a.sorted_node;
+	const long long ntiles = (a.npairs + PART - 1) / PART;
+	for (long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t + 1 < ntiles;
+	     t += ((long long)gridDim.x * blockDim.x) >> 5)   // warp-uniform
+	{
+		const long long tb = t * PART, te = tb + PART;
+		const uint32_t n = __ldg(key + te - 1);
+		const bool covers = __ldg(key + tb) == n;
+		if (__ldg(key + te) != n || (covers && tb > 0 && __ldg(key + tb - 1) == n)) continue;
+		long long last = t;   // the tile of the node's last pair
+		for (unsigned on = FULL; on == FULL;)
 		{
-			const int o = lane + 32 * r;
-			if (o < TD) gs[(size_t)n * TD + o] = acc[r];
+			const long long u = last + 1 + lane;
+			on = __ballot_sync(FULL, u < ntiles && __ldg(key + u * PART) == n);   // a run of low lanes
+			last += __popc(on);
 		}
+		for (int o = lane; o < a.TD; o += 32)
+		{
+			double s = a.part[(size_t)(2 * t + (covers ? 0 : 1)) * a.TD + o];
+#pragma unroll 4
+			for (long long u = t + 1; u <= last; u++) s += a.part[(size_t)(2 * u) * a.TD + o];
+			a.gs[(size_t)n * a.TD + o] = s;
+		}
+	}
+}
+
+// dL/dx from the pairs' cs * w: one warp per point.
+__global__ void __launch_bounds__(BLOCK) bwd_dx_kernel(const __grid_constant__ BwdArgs a)
+{
+	extern __shared__ double smem[];
+	const int lane = threadIdx.x & 31;
+	double* xs = smem + (threadIdx.x >> 5) * 3 * a.dim;
+	double* gxs = xs + a.dim;
+	const GridDesc& G = a.G;
+	for (;;)
+	{
+		long long p = 0;
+		if (lane == 0) p = (long long)atomicAdd(a.counter, 1ull);
+		p = __shfl_sync(FULL, p, 0);
+		if (p >= a.npts) break;
+		for (int k = lane; k < a.dim; k += 32) { xs[k] = a.x[(size_t)p * a.dim + k]; gxs[k] = 0.0; gxs[a.dim + k] = 0.0; }
+		__syncwarp();
+		const long long b = a.pair_off[p], e = a.pair_off[p + 1];
+		for (long long q = b; q < e; q += 32)
+		{
+			const int m = (int)min(32ll, e - q);
+			uint4 r = make_uint4(0u, 0u, 0u, 0u);
+			double csw = 0.0;
+			if (lane < m)
+			{
+				r = __ldg(G.rec + __ldg(a.pair_node + q + lane));
+				csw = a.pair_val[q + lane].w;
+			}
+			dx_pass(G, xs, gxs, a.dim, r.y, r.z & 0xffu, csw, m, lane);
+		}
+		__syncwarp();
+		for (int k = lane; k < a.dim; k += 32) a.gx[(size_t)p * a.dim + k] = gxs[k] + gxs[a.dim + k];
+		__syncwarp();
 	}
 }
 
@@ -1963,6 +2289,14 @@ size_t fwd_smem(int precision, int dim, bool descent = false)
 {
 	if (precision != SGI_FP32C) return (size_t)WARPS * hit_stride(dim) * sizeof(double);
 	return (size_t)WARPS * (descent ? desc_stride(dim) : list_stride(dim)) * sizeof(double);
+}
+
+template <int R>
+void (*nodes_kernel(bool dot, bool vec))(BwdArgs)
+{
+	if (R == 1) vec = false;   // one column per lane either way
+	return dot ? (vec ? bwd_nodes_kernel<R, true, R != 1> : bwd_nodes_kernel<R, true, false>)
+	           : (vec ? bwd_nodes_kernel<R, false, R != 1> : bwd_nodes_kernel<R, false, false>);
 }
 
 int pick_R(int cols)
@@ -3073,7 +3407,8 @@ extern "C" int sgi_interpolate_host(int ngrids, const sgi_grid_t* grids, const l
 
 namespace {
 
-int count_terms(sgi_grid_t g, long long npts, const double* x, long long* counts, long long* classes, void* stream)
+int count_terms(sgi_grid_t g, long long npts, const double* x, long long* counts, long long* classes, void* stream,
+	bool any = false)
 {
 	DeviceGuard guard(g->device);
 	DeviceWork* W = nullptr;
@@ -3087,12 +3422,12 @@ int count_terms(sgi_grid_t g, long long npts, const double* x, long long* counts
 	cudaStream_t s = (cudaStream_t)stream;
 	CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
 	const size_t smem = (size_t)WARPS * g->dim * sizeof(double);
-	void (*kern)(FwdArgs, long long*, long long*) = classes ? count_kernel<true> : count_kernel<false>;
+	void (*kern)(FwdArgs, long long*, long long*, bool) = classes ? count_kernel<true> : count_kernel<false>;
 	if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 	int blocks = 0;
 	rc = occupancy_grid(kern, smem, W->sms, &blocks);
 	if (rc) return rc;
-	kern<<<blocks, BLOCK, smem, s>>>(a, counts, classes);
+	kern<<<blocks, BLOCK, smem, s>>>(a, counts, classes, any);
 	CUDA_TRY(cudaGetLastError());
 	return SGI_OK;
 }
@@ -3136,83 +3471,100 @@ extern "C" int sgi_backward(sgi_grid_t g, long long npts, const double* x, const
 		gsurplus = nullptr;
 	}
 	if (npts == 0) return SGI_OK;
+	if (!gx && !gsurplus) return SGI_OK;
 	const int R = pick_R(g->TD);
-	void (*pk)(BwdArgs) = R == 1 ? bwd_points_kernel<1> : R == 2 ? bwd_points_kernel<2> : R == 4 ? bwd_points_kernel<4> : bwd_points_kernel<8>;
-	const size_t smem = (size_t)WARPS * 2 * g->dim * sizeof(double);
-	if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-	int blocks = 0;
-	rc = occupancy_grid(pk, smem, W->sms, &blocks);
-	if (rc) return rc;
-
 	BwdArgs a;
 	memset(&a, 0, sizeof(a));
 	a.G = desc_of(g, 0);
-	a.x = x; a.gout = gout; a.gx = gx; a.npts = npts; a.dim = g->dim; a.TD = g->TD;
+	a.x = x; a.gout = gout; a.gx = gx; a.gs = gsurplus; a.npts = npts; a.dim = g->dim; a.TD = g->TD;
+	// a persistent launch over `items` warp-sized work items
+	auto launch = [&](void (*kern)(BwdArgs), size_t smem, long long items) -> int
+	{
+		if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+		int blocks = 0;
+		int e = occupancy_grid(kern, smem, W->sms, &blocks);
+		if (e) return e;
+		blocks = (int)std::min<long long>(blocks, (items + WARPS - 1) / WARPS);
+		a.counter = W->counters + (W->next.fetch_add(1) % NCOUNTERS);
+		CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream));
+		kern<<<std::max(blocks, 1), BLOCK, smem, stream>>>(a);
+		CUDA_TRY(cudaGetLastError());
+		g_stats.kernels++;
+		return SGI_OK;
+	};
+	if (!gsurplus)
+	{
+		void (*pk)(BwdArgs) = R == 1 ? bwd_points_kernel<1> : R == 2 ? bwd_points_kernel<2> : R == 4 ? bwd_points_kernel<4> : bwd_points_kernel<8>;
+		g_stats.points = npts;
+		return launch(pk, (size_t)WARPS * bwd_stride(g->dim) * sizeof(double), npts);
+	}
 
 	// scratch (stream-ordered allocations from the device's pool)
 	cudaMemPool_t pool = nullptr;
 	rc = scratch_pool(W, g->device, &pool);
 	if (rc) return rc;
-	long long* counts = nullptr;
-	long long* offs = nullptr;
-	uint32_t *pn = nullptr, *node_sorted = nullptr;
-	PairVal *pv = nullptr, *val_sorted = nullptr;
-	void* tmp = nullptr;
-	long long npairs = 0;
-	auto cleanup = [&]()
+	std::vector<void*> held;
+	auto cleanup = [&]() { for (void* q : held) cudaFreeAsync(q, stream); held.clear(); };
+	auto take = [&](auto** dst, size_t bytes) -> cudaError_t
 	{
-		cudaFreeAsync(counts, stream); cudaFreeAsync(offs, stream); cudaFreeAsync(pn, stream);
-		cudaFreeAsync(pv, stream); cudaFreeAsync(val_sorted, stream); cudaFreeAsync(node_sorted, stream);
-		cudaFreeAsync(tmp, stream);
+		void* q = nullptr;
+		cudaError_t e = cudaMallocFromPoolAsync(&q, std::max<size_t>(bytes, 16), pool, stream);
+		if (e == cudaSuccess) held.push_back(q);
+		*dst = static_cast<std::remove_reference_t<decltype(**dst)>*>(q);
+		return e;
 	};
 #define BWD_TRY(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) { cleanup(); \
 	return fail(SGI_E_CUDA, "%s failed: %s", #call, cudaGetErrorString(e_)); } } while (0)
-	if (gsurplus)
+#define BWD_RUN(call) do { rc = (call); if (rc) { cleanup(); return rc; } } while (0)
+	long long* counts = nullptr;
+	long long* offs = nullptr;
+	char* tmp = nullptr;
+	long long npairs = 0;
+	BWD_TRY(take(&counts, sizeof(long long) * (npts + 1)));
+	BWD_TRY(take(&offs, sizeof(long long) * (npts + 1)));
+	BWD_TRY(cudaMemsetAsync(counts + npts, 0, sizeof(long long), stream));
+	BWD_RUN(count_terms(g, npts, x, counts, nullptr, stream, true));
+	size_t tb = 0;
+	BWD_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, counts, offs, npts + 1, stream));
+	BWD_TRY(take(&tmp, tb));
+	BWD_TRY(cub::DeviceScan::ExclusiveSum(tmp, tb, counts, offs, npts + 1, stream));
+	BWD_TRY(cudaMemcpyAsync(&npairs, offs + npts, sizeof(long long), cudaMemcpyDeviceToHost, stream));
+	BWD_TRY(cudaStreamSynchronize(stream));
+	if (npairs > 0x7fffffffll) { cleanup(); return fail(SGI_E_RANGE, "%lld active pairs exceed 2^31", npairs); }
+	a.npairs = npairs;
+	a.pair_off = offs;
+	uint32_t *node_sorted = nullptr, *idx_sorted = nullptr;
+	const long long ntiles = (npairs + PART - 1) / PART;
+	BWD_TRY(take(&a.pair_node, 4 * (size_t)npairs));
+	BWD_TRY(take(&a.pair_val, sizeof(PairVal) * (size_t)npairs));
+	BWD_TRY(take(&a.pair_idx, 4 * (size_t)npairs));
+	BWD_TRY(take(&node_sorted, 4 * (size_t)npairs));
+	BWD_TRY(take(&idx_sorted, 4 * (size_t)npairs));
+	BWD_TRY(take(&a.part, sizeof(double) * 2 * (size_t)ntiles * g->TD));
+	BWD_RUN(launch(bwd_list_kernel, (size_t)WARPS * hit_stride(g->dim) * sizeof(double), npts));
+	// stable radix sort by node: each node's pairs stay in point order
+	int endbit = 1;
+	while (endbit < 32 && (1ll << endbit) <= (long long)g->nno) endbit++;
+	if (npairs)
 	{
-		BWD_TRY(cudaMallocFromPoolAsync((void**)&counts, sizeof(long long) * (npts + 1), pool, stream));
-		BWD_TRY(cudaMallocFromPoolAsync((void**)&offs, sizeof(long long) * (npts + 1), pool, stream));
-		BWD_TRY(cudaMemsetAsync(counts + npts, 0, sizeof(long long), stream));
-		rc = sgi_active_count(g, npts, x, counts, stream);
-		if (rc) { cleanup(); return rc; }
-		size_t tb = 0;
-		BWD_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, counts, offs, npts + 1, stream));
-		BWD_TRY(cudaMallocFromPoolAsync(&tmp, tb, pool, stream));
-		BWD_TRY(cub::DeviceScan::ExclusiveSum(tmp, tb, counts, offs, npts + 1, stream));
-		BWD_TRY(cudaMemcpyAsync(&npairs, offs + npts, sizeof(long long), cudaMemcpyDeviceToHost, stream));
-		BWD_TRY(cudaStreamSynchronize(stream));
-		cudaFreeAsync(tmp, stream); tmp = nullptr;
-		if (npairs > 0x7fffffffll) { cleanup(); return fail(SGI_E_RANGE, "%lld active pairs exceed 2^31", npairs); }
-		const size_t np = (size_t)std::max(npairs, 1ll);
-		BWD_TRY(cudaMallocFromPoolAsync((void**)&pn, 4 * np, pool, stream));
-		BWD_TRY(cudaMallocFromPoolAsync((void**)&pv, sizeof(PairVal) * np, pool, stream));
-		a.pair_off = offs; a.pair_node = pn; a.pair_val = pv;
+		BWD_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, a.pair_node, node_sorted, a.pair_idx, idx_sorted, (int)npairs, 0, endbit, stream));
+		BWD_TRY(take(&tmp, tb));
+		BWD_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, a.pair_node, node_sorted, a.pair_idx, idx_sorted, (int)npairs, 0, endbit, stream));
 	}
-	a.counter = W->counters + (W->next.fetch_add(1) % NCOUNTERS);
-	BWD_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream));
-	pk<<<blocks, BLOCK, smem, stream>>>(a);
-	BWD_TRY(cudaGetLastError());
-	g_stats.kernels++;
-	if (gsurplus)
-	{
-		const size_t np = (size_t)std::max(npairs, 1ll);
-		BWD_TRY(cudaMallocFromPoolAsync((void**)&val_sorted, sizeof(PairVal) * np, pool, stream));
-		BWD_TRY(cudaMallocFromPoolAsync((void**)&node_sorted, 4 * np, pool, stream));
-		// stable radix sort by node: each node's pairs stay in point order
-		size_t tb = 0;
-		int endbit = 1;
-		while (endbit < 32 && (1ll << endbit) <= (long long)g->nno) endbit++;
-		BWD_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, pn, node_sorted, pv, val_sorted, (int)npairs, 0, endbit, stream));
-		BWD_TRY(cudaMallocFromPoolAsync(&tmp, tb, pool, stream));
-		BWD_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, pn, node_sorted, pv, val_sorted, (int)npairs, 0, endbit, stream));
-		void (*sk)(const uint32_t*, const PairVal*, long long, const double*, double*, int, int) =
-			R == 1 ? bwd_surplus_kernel<1> : R == 2 ? bwd_surplus_kernel<2> : R == 4 ? bwd_surplus_kernel<4> : bwd_surplus_kernel<8>;
-		sk<<<W->sms * 8, BLOCK, 0, stream>>>(node_sorted, val_sorted, npairs, gout, gsurplus, g->nno, g->TD);
-		BWD_TRY(cudaGetLastError());
-		g_stats.kernels += 1;   // and the library's radix sort
-	}
+	a.sorted_node = node_sorted;
+	a.sorted_idx = idx_sorted;
+	// gout rows are read 16 bytes at a time where they all start on 16 bytes
+	const bool vec = g->TD % 2 == 0 && (uintptr_t)gout % 16 == 0;
+	void (*nk)(BwdArgs) = R == 1 ? nodes_kernel<1>(gx, vec) : R == 2 ? nodes_kernel<2>(gx, vec)
+		: R == 4 ? nodes_kernel<4>(gx, vec) : nodes_kernel<8>(gx, vec);
+	BWD_TRY(cudaMemsetAsync(gsurplus, 0, sizeof(double) * (size_t)g->nno * g->TD, stream));   // nodes without pairs
+	if (ntiles) BWD_RUN(launch(nk, 0, ntiles));
+	if (ntiles > 1) BWD_RUN(launch(bwd_join_kernel, 0, ntiles));
+	if (gx) BWD_RUN(launch(bwd_dx_kernel, (size_t)WARPS * 3 * g->dim * sizeof(double), npts));
 	cleanup();
 	g_stats.points = npts;
 	return SGI_OK;
+#undef BWD_RUN
 #undef BWD_TRY
 }
 

@@ -1,0 +1,48 @@
+"""Backward kernels at the edges of their tiles: the pairs sorted by node are
+cut every 1,024 (nodes that begin, end or span several tiles, tiles of one
+node, a last tile of a few pairs), lists of 32 hits, row widths around the
+lane layout, one or two pairs per list, both gradients or either, against the
+oracle's gradient (tolerances of the other gradient tests) and, for either
+gradient alone, bit for bit against both."""
+import numpy as np
+import pytest
+
+import hddm_b200 as H
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("td", [1, 31, 33, 64, 65, 118, 129, 256])
+@pytest.mark.parametrize("dim,nno,npts", [(3, 5, 3), (2, 1, 1024), (3, 9, 1500), (10, 300, 700), (30, 3000, 257)])
+def test_backward_tiles(cuda, dim, nno, npts, td):
+    import torch
+    hg = H.HostGrid.adaptive(dim, nno, td, seed=dim + td)
+    X = H.gen_points(dim, npts, kind=0, seed=1, kink_reject=1e-6)
+    C = np.random.default_rng(2).standard_normal((npts, td))
+    g = H.Grid(hg)
+    x, c = torch.from_numpy(X).cuda(), torch.from_numpy(C).cuda()
+    gx, gs = H.backward(g, x, c)
+    ox, os_ = O.Gold(*hg.arrays()).gradient(X, C)
+    assert np.abs(gx.cpu().numpy() - ox).max() <= 1e-10 * (np.abs(ox).max() + 1e-300)
+    assert np.abs(gs.cpu().numpy() - os_).max() <= 1e-12 * (np.abs(os_).max() + 1e-300)
+    assert torch.equal(H.backward(g, x, c, want_surplus=False)[0], gx)
+    assert torch.equal(H.backward(g, x, c, want_x=False)[1], gs)
+
+
+def test_backward_point_outside_every_support(cuda):
+    """A NaN coordinate leaves its nodes inactive; the others still count, in
+    both entry forms, and no other point's gradient changes."""
+    import torch
+    hg = H.HostGrid.adaptive(10, 500, 40, seed=3)
+    X = H.gen_points(10, 100, kind=0, seed=4, kink_reject=1e-6)
+    C = np.random.default_rng(5).standard_normal((100, 40))
+    g = H.Grid(hg)
+    ref = H.backward(g, torch.from_numpy(X).cuda(), torch.from_numpy(C).cuda())[0]
+    X[31, 2] = np.nan
+    x, c = torch.from_numpy(X).cuda(), torch.from_numpy(C).cuda()
+    gx, gs = H.backward(g, x, c)
+    only = H.backward(g, x, c, want_surplus=False)[0]
+    assert torch.equal(gx, only) and bool(torch.isfinite(gx).all()) and bool(torch.isfinite(gs).all())
+    keep = torch.arange(100, device="cuda") != 31
+    assert torch.equal(gx[keep], ref[keep])
