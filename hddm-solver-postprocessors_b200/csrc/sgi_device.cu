@@ -145,19 +145,20 @@ __device__ __forceinline__ int find_grid(const FwdArgs& a, long long p)
 }
 
 // Product of a hit node's hats in dimension order (the gold loop's `temp`).
-// Components are fetched four at a time, so a node costs one memory round
-// trip per four components instead of one per component.
+// Components are fetched eight at a time, so a node costs one memory round
+// trip per eight components instead of one per component.
 __device__ __forceinline__ double node_weight(const GridDesc& G, const double* xs, uint32_t cptr, uint32_t ncomp)
 {
+	constexpr int NB = 8;
 	double w = 1.0;
-	for (uint32_t c0 = 0; c0 < ncomp; c0 += 4)
+	for (uint32_t c0 = 0; c0 < ncomp; c0 += NB)
 	{
-		uint2 cp[4];
+		uint2 cp[NB];
 #pragma unroll
-		for (int q = 0; q < 4; q++)
+		for (int q = 0; q < NB; q++)
 			cp[q] = c0 + q < ncomp ? __ldg(G.comps + cptr + c0 + q) : make_uint2(0u, 0u);
 #pragma unroll
-		for (int q = 0; q < 4; q++)
+		for (int q = 0; q < NB; q++)
 			if (c0 + q < ncomp) w = __dmul_rn(w, hat(xs[cp[q].x], cp[q].y));
 	}
 	return w;
@@ -451,19 +452,67 @@ __device__ __forceinline__ void load_row(const float* row, int o, bool in, float
 	else d[0] = in ? __ldg(row + o) : 0.f;
 }
 
-// A listed hit of the FP64 form.  Until its weight is known, `w` holds its
-// component range: {first component, component count} in two 32-bit words.
+// A lane's E neighbouring doubles of a row.  Volatile, so that a group's loads
+// are issued together, ahead of the adds: left to the compiler, loads moved
+// down to their uses and a group's round trips followed one another.
+template <int E>
+__device__ __forceinline__ void load_ahead(const double* row, double* d)
+{
+	if (E == 2) asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(d[0]), "=d"(d[E - 1]) : "l"(row));
+	else asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(d[0]) : "l"(row));
+}
+
+// A listed hit.  Until its weight is known, `w` holds two words of its record:
+// its first component and {component count, flags, ...}.
 struct __align__(16) Hit
 {
 	double w;
 	uint32_t node, pad;
 };
 
+__device__ __forceinline__ Hit listed_hit(uint32_t node, const uint4& rec)
+{
+	Hit t;
+	t.w = __hiloint2double((int)rec.z, (int)rec.y);
+	t.node = node;
+	t.pad = 0u;
+	return t;
+}
+__device__ __forceinline__ uint32_t hit_cptr(const Hit& h) { return (uint32_t)__double2loint(h.w); }
+__device__ __forceinline__ uint32_t hit_flags(const Hit& h) { return (uint32_t)__double2hiint(h.w); }
+__device__ __forceinline__ uint32_t hit_ncomp(const Hit& h) { return hit_flags(h) & 0xffu; }
+
 // Hits a warp lists before it takes their weights and rows: a window adds at
 // most 32 to a list that holds fewer than 32.
 constexpr int HCAP = 64;
 
 __host__ __device__ __forceinline__ int hit_stride(int dim) { return 2 * HCAP + ((dim + 1) & ~1); }
+
+// Walks nodes [lo, hi) for the point in xs (see traverse) and hands its hits
+// over in lists of at most 32, in index order: on_list(m), the list being
+// hits[0 .. m).
+template <class OnList>
+__device__ __forceinline__ void walk_lists(const GridDesc& G, const double* xs, Hit* hits, int lane, int lo, int hi,
+	unsigned pathmask, int clen, OnList&& on_list)
+{
+	int n = 0;
+	traverse<false>(G, xs, lane, lo, hi, [&](unsigned mask, int n0, double, const uint4& r, float)
+	{
+		if ((mask >> lane) & 1u) hits[n + __popc(mask & ((1u << lane) - 1u))] = listed_hit((uint32_t)(n0 + lane), r);
+		n += __popc(mask);
+		if (n >= 32)
+		{
+			__syncwarp();
+			on_list(32);
+			n -= 32;
+			__syncwarp();
+			if (lane < n) hits[lane] = hits[32 + lane];
+			__syncwarp();
+		}
+	}, nullptr, pathmask, clen);
+	__syncwarp();
+	if (n) on_list(n);
+}
 
 // FP64 form.  The walk only lists its hits (a window of 32 nodes holds two or
 // three of them); once 32 are listed, lane k takes hit k's weight, all lanes
@@ -520,19 +569,15 @@ __global__ void __launch_bounds__(BLOCK, 4) fwd_f64_kernel(const __grid_constant
 			}
 		if (ok)
 		{
-			const double* s64l = G.s64 + a.o_begin + out_col<E>(0, lane);
 			const uint32_t ld = (uint32_t)G.ld;
-			const int room = G.ld - a.o_begin - out_col<E>(0, lane);   // columns of a row from this lane's first
-			int n = 0;
-			// the first m <= 32 listed hits
-			auto take = [&](int m)
+			// columns past the row's end read this lane's first instead (their sums are not stored)
+			uint32_t at[V];
+#pragma unroll
+			for (int v = 0; v < V; v++) at[v] = a.o_begin + out_col<E>(v, lane) < G.ld ? v * 32 * E : 0;
+			const double* s64l = G.s64 + (a.o_begin + out_col<E>(0, lane) < G.ld ? a.o_begin + out_col<E>(0, lane) : 0);
+			walk_lists(G, xs, hits, lane, lo, hi, pathmask, a.chain_len[gi], [&](int m)
 			{
-				__syncwarp();
-				if (lane < m)
-				{
-					const double t = hits[lane].w;
-					hits[lane].w = node_weight(G, xs, (uint32_t)__double2loint(t), (uint32_t)__double2hiint(t));
-				}
+				if (lane < m) hits[lane].w = node_weight(G, xs, hit_cptr(hits[lane]), hit_ncomp(hits[lane]));
 				__syncwarp();
 				int h = 0;
 				for (; h + QH <= m; h += QH)
@@ -543,7 +588,7 @@ __global__ void __launch_bounds__(BLOCK, 4) fwd_f64_kernel(const __grid_constant
 					{
 						const double* row = s64l + (size_t)hits[h + q].node * ld;
 #pragma unroll
-						for (int v = 0; v < V; v++) load_row<E>(row, v * 32 * E, v * 32 * E < room, sq[q][v]);
+						for (int v = 0; v < V; v++) load_ahead<E>(row + at[v], sq[q][v]);
 					}
 #pragma unroll
 					for (int q = 0; q < QH; q++)
@@ -563,7 +608,7 @@ __global__ void __launch_bounds__(BLOCK, 4) fwd_f64_kernel(const __grid_constant
 					{
 						const double* row = s64l + (size_t)hits[min(h + q, m - 1)].node * ld;
 #pragma unroll
-						for (int v = 0; v < V; v++) load_row<E>(row, v * 32 * E, v * 32 * E < room && h + q < m, sq[q][v]);
+						for (int v = 0; v < V; v++) load_ahead<E>(row + at[v], sq[q][v]);
 					}
 #pragma unroll
 					for (int q = 0; q < QH; q++)
@@ -576,28 +621,7 @@ __global__ void __launch_bounds__(BLOCK, 4) fwd_f64_kernel(const __grid_constant
 							for (int e = 0; e < E; e++) acc[v][e] = __dadd_rn(acc[v][e], __dmul_rn(wq, sq[q][v][e]));
 					}
 				}
-			};
-			traverse<false>(G, xs, lane, lo, hi, [&](unsigned mask, int n0, double, const uint4& r, float)
-			{
-				if ((mask >> lane) & 1u)
-				{
-					Hit t;
-					t.w = __hiloint2double((int)(r.z & 0xffu), (int)r.y);
-					t.node = (uint32_t)(n0 + lane);
-					t.pad = 0u;
-					hits[n + __popc(mask & ((1u << lane) - 1u))] = t;
-				}
-				n += __popc(mask);
-				if (n >= 32)
-				{
-					take(32);
-					n -= 32;
-					__syncwarp();
-					if (lane < n) hits[lane] = hits[32 + lane];
-					__syncwarp();
-				}
-			}, nullptr, pathmask, a.chain_len[gi]);
-			if (n) take(n);
+			});
 		}
 #pragma unroll
 		for (int v = 0; v < V; v++)
@@ -1251,6 +1275,63 @@ constexpr int CDEPTH = 32;
 
 __host__ __device__ __forceinline__ int cols_stride(int dim) { return CLIST + CLIST / 2 + ((dim + 1) & ~1); }
 
+// Whether the FP32C form keeps a term of this node and weight.
+__device__ __forceinline__ bool keeps_term(const GridDesc& G, uint32_t flags, float rowmax, double w)
+{
+	const float bound = fabsf(__double2float_rn(w)) * rowmax;
+	return ((flags & NODE_COARSE) && bound >= G.big_below) || bound >= G.skip_below;
+}
+
+// Output `col` of a point, walked and added by this warp alone (lane l's
+// column is l's own): phase 2's way with a point whose lists found no room.
+// lw, ln: CLIST entries of shared memory.
+template <int DEPTH>
+__device__ __forceinline__ double walk_column(const GridDesc& G, const double* xs, double* lw, uint32_t* ln, int lane,
+	int col, bool cin)
+{
+	double acc = 0.0;
+	int n = 0;
+	// list entries [0, cnt) in order
+	auto drain = [&](int cnt)
+	{
+		for (int b = 0; b < cnt; b += DEPTH)
+		{
+			double sv[DEPTH];
+#pragma unroll
+			for (int q = 0; q < DEPTH; q++)
+				sv[q] = (b + q < cnt && cin) ? __ldg(G.s64 + (size_t)ln[b + q] * G.ld + col) : 0.0;
+#pragma unroll
+			for (int q = 0; q < DEPTH; q++)
+			{
+				if (b + q >= cnt) break;   // warp-uniform
+				acc = __dadd_rn(acc, __dmul_rn(lw[b + q], sv[q]));
+			}
+		}
+	};
+	traverse<false>(G, xs, lane, 0, G.nno, [&](unsigned mask, int n0, double w, const uint4& r, float rm)
+	{
+		bool keep = (mask >> lane) & 1u;
+		if (keep && G.rowmax) keep = keeps_term(G, r.z, rm, w);
+		const unsigned km = __ballot_sync(FULL, keep);
+		if (keep)
+		{
+			const int pos = n + __popc(km & ((1u << lane) - 1u));
+			ln[pos] = (uint32_t)(n0 + lane);
+			lw[pos] = w;
+		}
+		n += __popc(km);   // below CLIST - 32 before, below CLIST after
+		__syncwarp();
+		if (n >= CLIST - 32)
+		{
+			drain(n);
+			n = 0;
+			__syncwarp();
+		}
+	});
+	if (n) drain(n);
+	return acc;
+}
+
 __global__ void __launch_bounds__(BLOCK) fwd_f64_cols_kernel(const __grid_constant__ FwdArgs a)
 {
 	extern __shared__ double smem[];
@@ -1273,87 +1354,59 @@ __global__ void __launch_bounds__(BLOCK) fwd_f64_cols_kernel(const __grid_consta
 		const bool cin = col < cols;
 		const GridDesc& G = a.g[find_grid(a, p)];
 		const bool ok = load_point(a, p, xs, lane);
-		double acc = 0.0;
-		int n = 0;
-		// list entries [0, cnt) in order
-		auto drain = [&](int cnt)
-		{
-			for (int b = 0; b < cnt; b += CDEPTH)
-			{
-				double sv[CDEPTH];
-#pragma unroll
-				for (int q = 0; q < CDEPTH; q++)
-					sv[q] = (b + q < cnt && cin) ? __ldg(G.s64 + (size_t)ln[b + q] * G.ld + a.o_begin + col) : 0.0;
-#pragma unroll
-				for (int q = 0; q < CDEPTH; q++)
-				{
-					if (b + q >= cnt) break;   // warp-uniform
-					acc = __dadd_rn(acc, __dmul_rn(lw[b + q], sv[q]));
-				}
-			}
-		};
-		if (ok)
-		{
-			traverse<false>(G, xs, lane, 0, G.nno, [&](unsigned mask, int n0, double w, const uint4&, float)
-			{
-				if ((mask >> lane) & 1u)
-				{
-					const int pos = n + __popc(mask & ((1u << lane) - 1u));
-					ln[pos] = (uint32_t)(n0 + lane);
-					lw[pos] = w;
-				}
-				n += __popc(mask);   // below CLIST - 32 before, below CLIST after
-				__syncwarp();
-				if (n >= CLIST - 32)
-				{
-					drain(n);
-					n = 0;
-					__syncwarp();
-				}
-			});
-			if (n) drain(n);
-		}
+		const double acc = ok ? walk_column<CDEPTH>(G, xs, lw, ln, lane, a.o_begin + col, cin) : 0.0;
 		if (cin)
 			a.out[(size_t)p * a.TD + a.o_begin + col] = ok ? acc : (G.nno ? __longlong_as_double(0x7ff8000000000000ll) : 0.0);
 		__syncwarp();
 	}
 }
 
-// Small FP64 batches in two phases.  A point's walk takes its windows one
-// after another, and its warps then wait on their rows a few at a time; with
-// few points most of the GPU idles.  Here the walk is spread over many warps
-// and the rows are staged in bulk; the arithmetic is the gold kernel's, in
-// its order (bit-identical to fwd_f64_kernel).
-// Phase 1 (walk_chunks_kernel): one warp per (point, chunk of LCS nodes)
-// walks the chunk from its start's ancestor chain (a table built with the
-// grid), lists the chunk's hits in index order with their gold-order weights,
-// and prefetches their surplus rows into the L2.  For the FP32C form (grid
-// descriptors with row maxima) it lists only the terms the FP32C kernels keep
-// (big terms, and others whose bound reaches the dropped-term bound); their
-// FP64 rows are then added exactly.
-// Phase 2 (fwd_f64_list_kernel): one warp per (point, 32 outputs) takes the
-// point's hits chunk after chunk, copies the rows of LDEPTH hits into shared
-// memory (cp.async, one double per lane per row) and then adds them in order.
-constexpr int LCS = 512;                   // nodes per phase-1 chunk
-constexpr int LDEPTH = 256;                // rows per phase-2 copy round
-constexpr int LBLOCK = 64;                 // phase-2 threads per block
+// Batches in two phases: the walk of a point takes its windows one after
+// another, and a warp that owns a point then waits on its rows a few at a
+// time; with fewer points than the GPU holds warps, or a few times as many,
+// most of it idles.  Here the walk is spread over many warps per point, and
+// the rows over many warps per point by columns; the arithmetic is the gold
+// kernel's, in its order (bit-identical to fwd_f64_kernel).
+// Phase 1 (walk_chunks_kernel): one warp per (point, node chunk) walks the
+// chunk from its start's ancestor chain (a table built with the grid) and
+// lists its hits in index order with their gold-order weights.  For the FP32C
+// form (grid descriptors with row maxima) it lists only the terms the FP32C
+// kernels keep (big terms, and others whose bound reaches the dropped-term
+// bound); their FP64 rows are then added exactly.
+// Phase 2: the rows of a point's hits are added chunk after chunk, for a few
+// points by one block per (point, 32 outputs) with rows through shared memory
+// (fwd_f64_stage_kernel), else by one warp per (point, 32 or 64 outputs) with
+// rows through registers (fwd_f64_gather_kernel).
+//
+// Lists: item i's `cnt` hits are at [off, off + cnt) of the node and weight
+// arrays.  When every (point, node) has room (`cursor` null), off is the
+// item's own share; else items take what they need from a common pool, and an
+// item that finds none left (HIT_OVER) leaves its point to phase 2 to walk.
+constexpr int LSTEP = 128;                 // nodes per entry of a grid's chain table; chunks are multiples of it
+constexpr int WBUF = 192;                  // hits a phase-1 warp lists in shared memory
 constexpr uint32_t HIT_BAD = 0xffffffffu;  // hit count of a point with a non-finite coordinate
+constexpr uint32_t HIT_OVER = 0xfffffffeu; // hit count of an item without room
 
-__host__ __device__ __forceinline__ int list_stride() { return LDEPTH * 32 + LDEPTH + LDEPTH / 2; }
+__host__ __device__ __forceinline__ int walk_stride(int dim) { return 2 * WBUF + ((dim + 1) & ~1); }
 
 struct ListArgs
 {
 	GridDesc g[MAXG];
-	const uint32_t* ctab[MAXG];  // per chunk k, 32 words: {chain length, chain node at depth 1..length}
+	const uint32_t* ctab[MAXG];  // per LSTEP nodes, 32 words: {chain length, chain node at depth 1..length}
 	long long ibeg[MAXG + 1];    // first (point, chunk) item of each grid; a point's items are consecutive
 	int nch[MAXG];               // chunks per grid
 	const double* x;
 	double* out;
-	uint32_t* hcnt;              // hits of item i: hcnt[i] (HIT_BAD for a non-finite point)
-	uint32_t* hnode;             //   their nodes and weights at [i * LCS, i * LCS + hcnt[i])
+	uint2* item;                 // {off, cnt} per item
+	uint32_t* hnode;
 	double* hw;
+	unsigned long long* cursor;  // entries taken from the pool, or null
+	unsigned long long* counter; // phase 1's items taken beyond one per warp, or null; phase 2's follows
+	long long cap;               // entries of hnode and hw
 	long long npts;
 	int ngrids, dim, TD;
+	int clen;                    // nodes per chunk
+	int prefetch;                // bring listed rows into the L2
 };
 static_assert(sizeof(ListArgs) <= 32764, "ListArgs exceeds the kernel parameter limit");
 
@@ -1364,21 +1417,40 @@ __device__ __forceinline__ int list_grid(const ListArgs& a, long long p)
 	return gi;
 }
 
-__global__ void __launch_bounds__(BLOCK) walk_chunks_kernel(const __grid_constant__ ListArgs a)
+__global__ void __launch_bounds__(BLOCK, 5) walk_chunks_kernel(const __grid_constant__ ListArgs a)
 {
 	extern __shared__ double smem[];
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
-	double* xs = smem + warp * a.dim;
-	const long long nitems = a.ibeg[a.ngrids];
-	for (long long it = (long long)blockIdx.x * WARPS + warp; it < nitems; it += (long long)gridDim.x * WARPS)
+	double* wbase = smem + warp * walk_stride(a.dim);
+	Hit* hits = reinterpret_cast<Hit*>(wbase);
+	double* xs = wbase + 2 * WBUF;
+	const uint32_t nitems = (uint32_t)a.ibeg[a.ngrids];
+	uint32_t it = blockIdx.x * WARPS + warp;
+	for (bool first = true;; first = false)
 	{
+		// the first items go by warp number, the others by a counter
+		if (!first)
+		{
+			if (!a.counter) break;
+			if (lane == 0) it = gridDim.x * WARPS + (uint32_t)atomicAdd(a.counter, 1ull);
+			it = __shfl_sync(FULL, it, 0);
+		}
+		if (it >= nitems) break;
 		int gi = 0;
-		while (gi + 1 < a.ngrids && a.ibeg[gi + 1] <= it) gi++;
+		while (gi + 1 < a.ngrids && a.ibeg[gi + 1] <= (long long)it) gi++;
 		const GridDesc& G = a.g[gi];
-		const long long loc = it - a.ibeg[gi];
-		const long long p = G.pt_begin + loc / a.nch[gi];
-		const int k = (int)(loc % a.nch[gi]);
+		const uint32_t loc = it - (uint32_t)a.ibeg[gi], nch = (uint32_t)a.nch[gi];
+		const long long p = G.pt_begin + loc / nch;
+		const int k = (int)(loc % nch);
+		// the chunk's first window comes in with the point and the chain
+		const uint32_t* ch = a.ctab[gi] + (size_t)k * (a.clen / LSTEP) * 32;
+		const uint32_t chain = __ldg(ch + lane);   // {length, node at depth 1 ..}
+		int lo = k * a.clen;
+		const int hi = (int)min((long long)G.nno, (long long)lo + a.clen);
+		if (lane < 4) asm volatile("prefetch.global.L1 [%0];" :: "l"(G.rec + min(lo + 8 * lane, hi - 1)));
+		else if (lane < 6) asm volatile("prefetch.global.L1 [%0];" :: "l"(G.aux + min(lo + 16 * (lane - 4), hi - 1)));
+		else if (lane == 6) asm volatile("prefetch.global.L1 [%0];" :: "l"(G.parent + lo));
 		bool finite = true;
 		for (int d = lane; d < a.dim; d += 32)
 		{
@@ -1387,149 +1459,414 @@ __global__ void __launch_bounds__(BLOCK) walk_chunks_kernel(const __grid_constan
 			finite &= isfinite(v);
 		}
 		__syncwarp();
-		uint32_t cnt = HIT_BAD;
+		uint2 res = make_uint2(0u, HIT_BAD);
 		if (__all_sync(FULL, finite))
 		{
-			cnt = 0;
-			const uint32_t* ch = a.ctab[gi] + (size_t)k * 32;
-			const int len = (int)__ldg(ch);
-			int lo = k * LCS;
-			const int hi = min(G.nno, lo + LCS);
-			const unsigned pathmask = chain_state_of([&](int d) { return __ldg(ch + 1 + d); }, len, G, xs, lane,
-			                                         nullptr, &lo);
-			uint32_t* hn = a.hnode + (size_t)it * LCS;
-			double* hv = a.hw + (size_t)it * LCS;
-			const int rowb = a.TD * 8;
+			const int len = (int)__shfl_sync(FULL, chain, 0);
+			// lane d >= 1 asks for the chain node at depth d, the word it holds
+			const unsigned pathmask = chain_state_of([&](int) { return chain; }, len, G, xs, lane, nullptr, &lo);
+			// the hits are counted, and listed as far as the buffer goes
+			int n = 0;
 			if (lo < hi)
-				traverse<false>(G, xs, lane, lo, hi, [&](unsigned mask, int n0, double w, const uint4& r, float rm)
+				traverse<false>(G, xs, lane, lo, hi, [&](unsigned mask, int n0, double, const uint4& r, float)
 				{
-					bool keep = (mask >> lane) & 1u;
-					if (keep && G.rowmax)
+					const int pos = n + __popc(mask & ((1u << lane) - 1u));
+					if (((mask >> lane) & 1u) && pos < WBUF) hits[pos] = listed_hit((uint32_t)(n0 + lane), r);
+					n += __popc(mask);
+				}, nullptr, pathmask, len);
+			unsigned long long off = (unsigned long long)it * a.clen;
+			if (a.cursor)
+			{
+				if (lane == 0 && n) off = atomicAdd(a.cursor, (unsigned long long)n);
+				off = __shfl_sync(FULL, off, 0);
+			}
+			if (n == 0) res = make_uint2(0u, 0u);
+			else if (off + n > (unsigned long long)a.cap) res = make_uint2(0u, HIT_OVER);
+			else
+			{
+				uint32_t kept = 0;
+				const int rowb = a.TD * 8;
+				auto emit = [&](const Hit* list, int m)
+				{
+					Hit h = list[min(lane, m - 1)];
+					double w = 0.0;
+					bool keep = lane < m;
+					if (keep)
 					{
-						const float bound = fabsf(__double2float_rn(w)) * rm;
-						keep = ((r.z & NODE_COARSE) && bound >= G.big_below) || bound >= G.skip_below;
+						float rm = 0.f;
+						if (G.rowmax) rm = __ldg(G.rowmax + h.node);
+						w = node_weight(G, xs, hit_cptr(h), hit_ncomp(h));
+						if (G.rowmax) keep = keeps_term(G, hit_flags(h), rm, w);
 					}
 					const unsigned km = __ballot_sync(FULL, keep);
 					if (keep)
 					{
-						const uint32_t pos = cnt + __popc(km & ((1u << lane) - 1u));
-						hn[pos] = (uint32_t)(n0 + lane);
-						hv[pos] = w;
-						const char* row = reinterpret_cast<const char*>(G.s64 + (size_t)(n0 + lane) * G.ld);
-						for (int b = 0; b < rowb; b += 128) asm volatile("prefetch.global.L2 [%0];" :: "l"(row + b));
+						const size_t e = (size_t)off + kept + __popc(km & ((1u << lane) - 1u));
+						a.hnode[e] = h.node;
+						a.hw[e] = w;
+						if (a.prefetch)
+						{
+							const char* row = reinterpret_cast<const char*>(G.s64 + (size_t)h.node * G.ld);
+							for (int b = 0; b < rowb; b += 128) asm volatile("prefetch.global.L2 [%0];" :: "l"(row + b));
+						}
 					}
-					cnt += __popc(km);
-				}, nullptr, pathmask, len);
+					kept += __popc(km);
+				};
+				__syncwarp();
+				if (n <= WBUF)
+					for (int b = 0; b < n; b += 32) emit(hits + b, min(32, n - b));
+				else
+					walk_lists(G, xs, hits, lane, lo, hi, pathmask, len, [&](int m) { emit(hits, m); });
+				res = make_uint2((uint32_t)off, kept);
+			}
 		}
-		if (lane == 0) a.hcnt[it] = cnt;
+		if (lane == 0) a.item[it] = res;
 		__syncwarp();
 	}
 }
 
-__global__ void __launch_bounds__(LBLOCK) fwd_f64_list_kernel(const __grid_constant__ ListArgs a)
+// Phase 2, rows through registers: one warp per (point, 32 * E outputs), QH
+// rows in flight; the next 32 list entries are loaded while 32 are added.
+// Bound by the longest point's round trips (1,500 points of up to 3,648 hits,
+// 118 outputs: 287 us with 8 rows of 64 outputs in flight, 226 with 16; 24
+// warps per SM of the one or 16 of the other).
+template <int E, int QH>
+__global__ void __launch_bounds__(BLOCK, E * QH > 16 ? 2 : 3) fwd_f64_gather_kernel(const __grid_constant__ ListArgs a)
 {
 	extern __shared__ double smem[];
 	const int lane = threadIdx.x & 31;
-	const int warp = threadIdx.x >> 5;
-	double* rows = smem + (size_t)warp * list_stride();
-	double* ew = rows + LDEPTH * 32;
-	uint32_t* en = reinterpret_cast<uint32_t*>(ew + LDEPTH);
-	const uint32_t rows_s = (uint32_t)__cvta_generic_to_shared(rows) + lane * 8u;
-	const int ncb = (a.TD + 31) / 32;
-	const long long nitems = a.npts * ncb;
-	for (long long it = (long long)blockIdx.x * (LBLOCK / 32) + warp; it < nitems;
-	     it += (long long)gridDim.x * (LBLOCK / 32))
+	double* wbase = smem + (threadIdx.x >> 5) * cols_stride(a.dim);
+	Hit* hits = reinterpret_cast<Hit*>(wbase);
+	const int ncb = (a.TD + 32 * E - 1) / (32 * E);
+	const uint32_t nitems = (uint32_t)(a.npts * ncb);
+	uint32_t it = blockIdx.x * WARPS + (threadIdx.x >> 5);
+	for (bool first = true;; first = false)
 	{
-		const long long p = it / ncb;
-		const int col = (int)(it % ncb) * 32 + lane;
-		const bool cin = col < a.TD;
+		if (!first)
+		{
+			if (!a.counter) break;
+			if (lane == 0) it = gridDim.x * WARPS + (uint32_t)atomicAdd(a.counter + 1, 1ull);
+			it = __shfl_sync(FULL, it, 0);
+		}
+		if (it >= nitems) break;
+		const long long p = it / (uint32_t)ncb;
+		const int col = (int)(it % (uint32_t)ncb) * 32 * E + lane * E;
 		const int gi = list_grid(a, p);
 		const GridDesc& G = a.g[gi];
 		const int nch = a.nch[gi];
 		const long long i0 = a.ibeg[gi] + (p - G.pt_begin) * nch;
+		const bool cin = col < G.ld;
 		const double* src = G.s64 + (cin ? col : 0);
-		double acc = 0.0;
-		bool ok = true;
-		// hits of chunks k0 .. k0 + 31: lane l holds chunk k0 + l's count c and
-		// the exclusive prefix excl; t of the group's T hits are taken
+		const uint32_t ld = (uint32_t)G.ld;
+		double acc[E];
+#pragma unroll
+		for (int e = 0; e < E; e++) acc[e] = 0.0;
+		bool bad = false, over = false;
+		// hits of items k0 .. k0 + 31: lane l holds item k0 + l's entries and
+		// the exclusive prefix of the counts; t of the group's T hits are taken
 		int k0 = -32;
-		uint32_t c = 0, excl = 0, T = 0, t = 0;
-		for (;;)
+		uint32_t off = 0, excl = 0, T = 0, t = 0;
+		// the next m <= 32 hits' nodes and weights, to lanes 0 .. m - 1
+		auto next = [&](uint32_t& nd, double& w) -> int
 		{
-			int m = 0;
-			while (m < LDEPTH)
+			while (t == T)
 			{
-				if (t == T)
+				k0 += 32;
+				if (k0 >= nch) return 0;
+				const uint2 v = k0 + lane < nch ? __ldg(a.item + i0 + k0 + lane) : make_uint2(0u, 0u);
+				bad = bad || __any_sync(FULL, v.y == HIT_BAD);
+				over = over || __any_sync(FULL, v.y == HIT_OVER);
+				if (bad || over) return 0;
+				off = v.x;
+				uint32_t incl = v.y;
+#pragma unroll
+				for (int s = 1; s < 32; s <<= 1)
 				{
-					k0 += 32;
-					if (k0 >= nch) break;
-					c = k0 + lane < nch ? __ldg(a.hcnt + i0 + k0 + lane) : 0u;
-					if (__any_sync(FULL, c == HIT_BAD)) { ok = false; break; }
-					uint32_t incl = c;
-#pragma unroll
-					for (int off = 1; off < 32; off <<= 1)
-					{
-						const uint32_t v = __shfl_up_sync(FULL, incl, off);
-						if (lane >= off) incl += v;
-					}
-					T = __shfl_sync(FULL, incl, 31);
-					excl = incl - c;
-					t = 0;
-					continue;
+					const uint32_t u = __shfl_up_sync(FULL, incl, s);
+					if (lane >= s) incl += u;
 				}
-				const uint32_t take = min(T - t, (uint32_t)(LDEPTH - m));
-				// list positions of hits t .. t + take - 1 first, then all their
-				// loads, then the stores: one round trip for the whole take
-				size_t e[LDEPTH / 32];
-#pragma unroll
-				for (int j = 0; j < LDEPTH / 32; j++)
-				{
-					const uint32_t h = t + (uint32_t)(j * 32 + lane);
-					// the chunk of hit h: the last lane whose prefix is at most h
-					int sl = 0;
-#pragma unroll
-					for (int step = 16; step >= 1; step >>= 1)
-					{
-						const uint32_t v = __shfl_sync(FULL, excl, sl + step);
-						if (v <= h) sl += step;
-					}
-					const uint32_t es = __shfl_sync(FULL, excl, sl);
-					e[j] = (size_t)(i0 + k0 + sl) * LCS + (h - es);
-				}
-				uint32_t nd[LDEPTH / 32];
-				double wv[LDEPTH / 32];
-#pragma unroll
-				for (int j = 0; j < LDEPTH / 32; j++)
-				{
-					const bool in = (uint32_t)(j * 32 + lane) < take;
-					nd[j] = in ? a.hnode[e[j]] : 0u;
-					wv[j] = in ? a.hw[e[j]] : 0.0;
-				}
-#pragma unroll
-				for (int j = 0; j < LDEPTH / 32; j++)
-					if ((uint32_t)(j * 32 + lane) < take)
-					{
-						en[m + j * 32 + lane] = nd[j];
-						ew[m + j * 32 + lane] = wv[j];
-					}
-				m += (int)take;
-				t += take;
+				T = __shfl_sync(FULL, incl, 31);
+				excl = incl - v.y;
+				t = 0;
 			}
-			if (!ok || m == 0) break;
-			__syncwarp();
-			if (cin)
+			const int m = (int)min(T - t, 32u);
+			const uint32_t h = t + (uint32_t)lane;
+			// the item of hit h: the last lane whose prefix is at most h
+			int sl = 0;
+#pragma unroll
+			for (int step = 16; step >= 1; step >>= 1)
 			{
-				for (int q = 0; q < m; q++)
-					asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
-					             :: "r"(rows_s + (uint32_t)q * 256u), "l"(src + (size_t)en[q] * G.ld) : "memory");
+				const uint32_t u = __shfl_sync(FULL, excl, sl + step);
+				if (u <= h) sl += step;
 			}
-			asm volatile("cp.async.wait_all;" ::: "memory");
+			const uint32_t es = __shfl_sync(FULL, excl, sl), os = __shfl_sync(FULL, off, sl);
+			nd = 0u;
+			w = 0.0;
+			if (lane < m)
+			{
+				nd = __ldg(a.hnode + (size_t)os + (h - es));
+				w = __ldg(a.hw + (size_t)os + (h - es));
+			}
+			t += (uint32_t)m;
+			return m;
+		};
+		uint32_t nd = 0u;
+		double w = 0.0;
+		int m = next(nd, w);
+		while (m)
+		{
 			__syncwarp();
-#pragma unroll 8
-			for (int q = 0; q < m; q++) acc = __dadd_rn(acc, __dmul_rn(ew[q], rows[q * 32 + lane]));
+			if (lane < m)
+			{
+				Hit h;
+				h.w = w; h.node = nd; h.pad = 0u;
+				hits[lane] = h;
+			}
+			__syncwarp();
+			const int mc = m;
+			m = next(nd, w);
+			if (bad || over) break;
+			int h = 0;
+			for (; h + QH <= mc; h += QH)
+			{
+				double sq[QH][E];
+#pragma unroll
+				for (int q = 0; q < QH; q++) load_ahead<E>(src + (size_t)hits[h + q].node * ld, sq[q]);
+#pragma unroll
+				for (int q = 0; q < QH; q++)
+				{
+					const double wq = hits[h + q].w;
+#pragma unroll
+					for (int e = 0; e < E; e++) acc[e] = __dadd_rn(acc[e], __dmul_rn(wq, sq[q][e]));
+				}
+			}
+			if (h < mc)
+			{
+				double sq[QH][E];
+#pragma unroll
+				for (int q = 0; q < QH; q++) load_ahead<E>(src + (size_t)hits[min(h + q, mc - 1)].node * ld, sq[q]);
+#pragma unroll
+				for (int q = 0; q < QH; q++)
+				{
+					if (h + q >= mc) break;   // warp-uniform
+					const double wq = hits[h + q].w;
+#pragma unroll
+					for (int e = 0; e < E; e++) acc[e] = __dadd_rn(acc[e], __dmul_rn(wq, sq[q][e]));
+				}
+			}
+		}
+		if (over && !bad)
+		{
+			double* xs = wbase + CLIST + CLIST / 2;
+			__syncwarp();
+			for (int d = lane; d < a.dim; d += 32) xs[d] = a.x[(size_t)p * a.dim + d];
+			__syncwarp();
+#pragma unroll
+			for (int e = 0; e < E; e++)
+				acc[e] = walk_column<8>(G, xs, wbase, reinterpret_cast<uint32_t*>(wbase + CLIST), lane, col + e, col + e < a.TD);
 			__syncwarp();
 		}
-		if (cin) a.out[(size_t)p * a.TD + col] = ok ? acc : (G.nno ? __longlong_as_double(0x7ff8000000000000ll) : 0.0);
+#pragma unroll
+		for (int e = 0; e < E; e++)
+			if (col + e < a.TD)
+				a.out[(size_t)p * a.TD + col + e] = !bad ? acc[e] : (G.nno ? __longlong_as_double(0x7ff8000000000000ll) : 0.0);
+		__syncwarp();
+	}
+}
+
+// Phase 2 through shared memory: one block per (point, 32 * NC outputs).  All
+// threads find the point's entries (a block-wide prefix sum over its items'
+// counts, then a search per hit); NP warps then copy the rows, SROWS to a
+// stage, into a ring of SRING stages (cp.async, 16 bytes each) while NC warps,
+// a lane per output, add the stage before.  A few points' time is one point's
+// chain of adds (8 cycles each) and the round trips before it: 192 rows in
+// flight add at 24 cycles a row (16 states of 23,000 nodes, one point each:
+// 17 us, where one warp that copied 256 rows, waited and added them took 49).
+constexpr int SITEMS = 1024;               // items per round
+
+// rows, weights, nodes, the items' prefixes and entries, a word per warp
+template <int NC, int SROWS, int SRING, int SENTRIES>
+constexpr size_t stage_smem() { return (size_t)SRING * SROWS * NC * 256 + SENTRIES * 12 + SITEMS * 8 + 64; }
+
+template <int NC, int NP, int SROWS, int SRING, int SENTRIES>
+__global__ void __launch_bounds__((NC + NP) * 32) fwd_f64_stage_kernel(const __grid_constant__ ListArgs a)
+{
+	constexpr int SB = (NC + NP) * 32;         // threads
+	constexpr int IPT = (SITEMS + SB - 1) / SB; // items per thread
+	extern __shared__ double smem[];
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	double* rows = smem;
+	double* ew = rows + SRING * SROWS * NC * 32;
+	uint32_t* en = reinterpret_cast<uint32_t*>(ew + SENTRIES);
+	uint32_t* ipre = en + SENTRIES;
+	uint32_t* ioff = ipre + SITEMS;
+	uint32_t* sums = ioff + SITEMS;
+	const uint32_t rows_s = (uint32_t)__cvta_generic_to_shared(rows);
+	const int ncg = (a.TD + 32 * NC - 1) / (32 * NC);
+	const uint32_t nitems = (uint32_t)(a.npts * ncg);
+	for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x)
+	{
+		const long long p = it / (uint32_t)ncg;
+		const int cb = (int)(it % (uint32_t)ncg) * 32 * NC, col = cb + tid;   // a consumer's output
+		const int gi = list_grid(a, p);
+		const GridDesc& G = a.g[gi];
+		const int nch = a.nch[gi];
+		const long long i0 = a.ibeg[gi] + (p - G.pt_begin) * nch;
+		double acc = 0.0;
+		bool bad = false, over = false;
+		for (int k0 = 0; k0 < nch; k0 += SITEMS)
+		{
+			// items k0 .. k0 + ni - 1: entries and the hits before them
+			const int ni = min(nch - k0, SITEMS);
+			uint2 v[IPT];
+			uint32_t mine = 0;
+			bool b = false, o = false;
+#pragma unroll
+			for (int j = 0; j < IPT; j++)
+			{
+				const int k = tid * IPT + j;
+				v[j] = k < ni ? __ldg(a.item + i0 + k0 + k) : make_uint2(0u, 0u);
+			}
+#pragma unroll
+			for (int j = 0; j < IPT; j++)
+			{
+				b = b || v[j].y == HIT_BAD;
+				o = o || v[j].y == HIT_OVER;
+				mine += v[j].y;
+			}
+			bad = __syncthreads_or(b);
+			over = __syncthreads_or(o);
+			if (bad || over) break;
+			uint32_t incl = mine;
+#pragma unroll
+			for (int s = 1; s < 32; s <<= 1)
+			{
+				const uint32_t u = __shfl_up_sync(FULL, incl, s);
+				if (lane >= s) incl += u;
+			}
+			if (lane == 31) sums[warp] = incl;
+			__syncthreads();
+			uint32_t before = incl - mine, T = 0;
+#pragma unroll
+			for (int s = 0; s < NC + NP; s++)
+			{
+				if (s < warp) before += sums[s];
+				T += sums[s];
+			}
+#pragma unroll
+			for (int j = 0; j < IPT; j++)
+			{
+				const int k = tid * IPT + j;
+				if (k < ni)
+				{
+					ipre[k] = before;
+					ioff[k] = v[j].x;
+				}
+				before += v[j].y;
+			}
+			__syncthreads();
+			for (uint32_t s0 = 0; s0 < T; s0 += SENTRIES)
+			{
+				const int M = (int)min(T - s0, (uint32_t)SENTRIES);
+				for (int e0 = 0; e0 < M; e0 += 4 * SB)
+				{
+					uint32_t nd[4];
+					double w[4];
+#pragma unroll
+					for (int j = 0; j < 4; j++)
+					{
+						const int e = e0 + j * SB + tid;
+						nd[j] = 0u;
+						w[j] = 0.0;
+						if (e < M)
+						{
+							// the item of hit s0 + e: the last with at most that many before it
+							const uint32_t h = s0 + (uint32_t)e;
+							int l = 0, r = ni;
+							while (r - l > 1)
+							{
+								const int c = (l + r) >> 1;
+								if (ipre[c] <= h) l = c;
+								else r = c;
+							}
+							const size_t at = (size_t)ioff[l] + (h - ipre[l]);
+							nd[j] = __ldg(a.hnode + at);
+							w[j] = __ldg(a.hw + at);
+						}
+					}
+#pragma unroll
+					for (int j = 0; j < 4; j++)
+					{
+						const int e = e0 + j * SB + tid;
+						if (e < M) { en[e] = nd[j]; ew[e] = w[j]; }
+					}
+				}
+				__syncthreads();
+				const int nst = (M + SROWS - 1) / SROWS;
+				// stage st's rows, by the copying warps (a commit per stage, empty past the last)
+				const int ptid = tid - NC * 32;
+				const int ch = ptid & (NC * 16 - 1);              // this thread's 16 bytes of a row
+				const bool cin = cb + 2 * ch < G.ld;
+				const double* src = G.s64 + (cin ? cb + 2 * ch : 0);
+				constexpr int RSTEP = NP * 32 / (NC * 16);        // rows copied at a time
+				auto issue = [&](int st)
+				{
+					if (st < nst)
+					{
+						const int cnt = min(SROWS, M - st * SROWS);
+						const uint32_t* n = en + st * SROWS;
+						const uint32_t dst = rows_s + (uint32_t)(st % SRING) * (SROWS * NC * 256) + (uint32_t)ch * 16u;
+#pragma unroll 8
+						for (int r = ptid / (NC * 16); r < cnt; r += RSTEP)
+							if (cin)
+								asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + (uint32_t)r * (NC * 256u)),
+									"l"(src + (size_t)n[r] * (uint32_t)G.ld) : "memory");
+					}
+					asm volatile("cp.async.commit_group;" ::: "memory");
+				};
+				if (warp >= NC)
+					for (int st = 0; st < SRING - 1; st++) issue(st);
+				for (int st = 0; st < nst; st++)
+				{
+					if (warp >= NC) asm volatile("cp.async.wait_group %0;" :: "n"(SRING - 2) : "memory");
+					__syncthreads();   // stage st has landed, stage st - 1 has been added
+					if (warp >= NC) issue(st + SRING - 1);
+					else
+					{
+						const double* r = rows + (size_t)(st % SRING) * (SROWS * NC * 32) + tid;
+						const double* w = ew + st * SROWS;
+						const int cnt = min(SROWS, M - st * SROWS);
+						int q = 0;
+						for (; q + 16 <= cnt; q += 16)
+						{
+							double t[16];
+#pragma unroll
+							for (int j = 0; j < 16; j++) t[j] = __dmul_rn(w[q + j], r[(q + j) * (NC * 32)]);
+#pragma unroll
+							for (int j = 0; j < 16; j++) acc = __dadd_rn(acc, t[j]);
+						}
+						for (; q < cnt; q++) acc = __dadd_rn(acc, __dmul_rn(w[q], r[q * (NC * 32)]));
+					}
+				}
+				if (warp >= NC) asm volatile("cp.async.wait_group 0;" ::: "memory");
+				__syncthreads();   // before the entries are replaced
+			}
+		}
+		if (over && !bad)
+		{
+			// items found no room: each consumer walks the point for its outputs
+			double* base = rows + (size_t)warp * cols_stride(a.dim);
+			if (warp < NC)
+			{
+				double* xs = base + CLIST + CLIST / 2;
+				for (int d = lane; d < a.dim; d += 32) xs[d] = a.x[(size_t)p * a.dim + d];
+				__syncwarp();
+				acc = walk_column<16>(G, xs, base, reinterpret_cast<uint32_t*>(base + CLIST), lane, col, col < a.TD);
+			}
+		}
+		if (warp < NC && col < a.TD)
+			a.out[(size_t)p * a.TD + col] = !bad ? acc : (G.nno ? __longlong_as_double(0x7ff8000000000000ll) : 0.0);
+		__syncthreads();
 	}
 }
 
@@ -1804,47 +2141,6 @@ __device__ __forceinline__ void dx_pass(const GridDesc& G, const double* xs, dou
 
 __host__ __device__ __forceinline__ int bwd_stride(int dim) { return HCAP * 2 + 3 * dim + (dim & 1); }
 
-// Walks point p's active nodes and hands them over in lists of at most 32 in
-// index order: on_list(m, hit) with lane k < m holding hit k (its component
-// range in w, see Hit).
-template <class OnList>
-__device__ __forceinline__ void walk_lists(const GridDesc& G, const double* xs, Hit* hits, int lane, OnList&& on_list)
-{
-	int n = 0;
-	auto take = [&](int m)
-	{
-		__syncwarp();
-		Hit h;
-		h.w = 0.0; h.node = 0u; h.pad = 0u;
-		if (lane < m) h = hits[lane];
-		on_list(m, h);
-	};
-	traverse<false>(G, xs, lane, 0, G.nno, [&](unsigned mask, int n0, double, const uint4& r, float)
-	{
-		if ((mask >> lane) & 1u)
-		{
-			Hit t;
-			t.w = __hiloint2double((int)(r.z & 0xffu), (int)r.y);
-			t.node = (uint32_t)(n0 + lane);
-			t.pad = 0u;
-			hits[n + __popc(mask & ((1u << lane) - 1u))] = t;
-		}
-		n += __popc(mask);
-		if (n >= 32)
-		{
-			take(32);
-			n -= 32;
-			__syncwarp();
-			if (lane < n) hits[lane] = hits[32 + lane];
-			__syncwarp();
-		}
-	});
-	if (n) take(n);
-}
-
-__device__ __forceinline__ uint32_t hit_cptr(const Hit& h) { return (uint32_t)__double2loint(h.w); }
-__device__ __forceinline__ uint32_t hit_ncomp(const Hit& h) { return (uint32_t)__double2hiint(h.w); }
-
 // dL/dx without dL/dsurplus: one warp per point, 32 hits at a time.
 template <int R>
 __global__ void __launch_bounds__(BLOCK, R == 8 ? 2 : 3) bwd_points_kernel(const __grid_constant__ BwdArgs a)
@@ -1866,8 +2162,9 @@ __global__ void __launch_bounds__(BLOCK, R == 8 ? 2 : 3) bwd_points_kernel(const
 		double g[R];
 		bwd_row<R, false>(a.gout + (size_t)p * a.TD, a.TD, lane, g);
 		__syncwarp();
-		walk_lists(G, xs, hits, lane, [&](int m, const Hit& h)
+		walk_lists(G, xs, hits, lane, 0, G.nno, 1u, 0, [&](int m)
 		{
+			const Hit h = hits[min(lane, m - 1)];
 			const double w = lane < m ? node_weight(G, xs, hit_cptr(h), hit_ncomp(h)) : 0.0;
 			const double cs = rows_dot<R>(G.s64, (uint32_t)G.ld, h.node, m, lane, g);
 			dx_pass(G, xs, gxs, a.dim, hit_cptr(h), hit_ncomp(h), cs * w, m, lane);
@@ -1896,10 +2193,11 @@ __global__ void __launch_bounds__(BLOCK) bwd_list_kernel(const __grid_constant__
 		for (int k = lane; k < a.dim; k += 32) xs[k] = a.x[(size_t)p * a.dim + k];
 		__syncwarp();
 		long long at = a.pair_off[p];
-		walk_lists(G, xs, hits, lane, [&](int m, const Hit& h)
+		walk_lists(G, xs, hits, lane, 0, G.nno, 1u, 0, [&](int m)
 		{
 			if (lane < m)
 			{
+				const Hit h = hits[lane];
 				a.pair_node[at + lane] = h.node;
 				a.pair_val[at + lane] = PairVal{ node_weight(G, xs, hit_cptr(h), hit_ncomp(h)), (uint32_t)p, 0u };
 				a.pair_idx[at + lane] = (uint32_t)(at + lane);
@@ -2350,10 +2648,11 @@ struct sgi_grid
 	std::vector<int> parent_h;
 	std::vector<uint32_t> skip_h, depth_h;
 	std::vector<uint32_t> gfirst_h, gcount_h, gcmin_h, gpmax_h;
-	// two-phase small batches: per chunk of LCS nodes, 32 words {length of
+	// two-phase batches: per LSTEP nodes, 32 words {length of
 	// the chunk start's ancestor chain, chain node at depth 1..length}
 	uint32_t* ctab = nullptr;
 	int nlch = 0;
+	double mean_active = 0.0;    // active nodes per point, mean over the unit cube
 	sgi_grid_info info{};
 };
 
@@ -2445,6 +2744,7 @@ struct GridImage
 	unsigned flags = 0;
 	int dim = 0, nno = 0, TD = 0, ld = 0, nlch = 0;
 	float skip_floor = 0.f, f16_floor = 0.f;
+	double mean_active = 0.0;
 	std::vector<uint32_t> rec, comps, coarse_index, aux, ctab, grp_a, grp_b, ninfo;
 	std::vector<uint16_t> s16;
 	std::vector<int> parent;
@@ -2488,15 +2788,32 @@ int build_image(const HostGrid& g, unsigned flags, GridImage& im)
 	const size_t nrow = (size_t)std::max(g.nno, 1);
 	im.rec = L.rec; im.comps = L.comps; im.coarse_index = L.lo_index; im.parent = L.parent; im.aux = L.aux;
 	im.parent_h = L.parent;
+	// a node's share of the unit cube is the product of its supports' lengths,
+	// (min(i, j + 1) - max(0, j - 1)) / i
+	for (int n = 0; n < g.nno; n++)
+	{
+		const uint32_t* r = &L.rec[4 * (size_t)n];
+		if (r[2] & NODE_DEAD) continue;
+		const uint32_t* c = L.comps.data() + 2 * (size_t)r[1];
+		double num = 1.0, den = 1.0;
+		for (uint32_t k = 0; k < (r[2] & 0xffu); k++)
+		{
+			const int i = (int)(c[2 * k + 1] & 0xffffu), j = (int)(c[2 * k + 1] >> 16);
+			if (i == 0) continue;
+			num *= std::max(0, std::min(i, j + 1) - std::max(0, j - 1));
+			den *= i;
+		}
+		if (den < 1e300) im.mean_active += num / den;
+	}
 	im.skip_h.resize(g.nno);
 	im.depth_h.resize(g.nno);
 	for (int n = 0; n < g.nno; n++) { im.skip_h[n] = L.rec[4 * (size_t)n]; im.depth_h[n] = L.aux[2 * (size_t)n + 1]; }
 	if (g.nno > 0)
 	{
-		im.nlch = (g.nno + LCS - 1) / LCS;
+		im.nlch = (g.nno + LSTEP - 1) / LSTEP;
 		im.ctab.assign((size_t)im.nlch * 32, 0u);
 		for (int k = 0; k < im.nlch; k++)
-			im.ctab[(size_t)k * 32] = (uint32_t)chain_at(&im, k * LCS, &im.ctab[(size_t)k * 32 + 1]);
+			im.ctab[(size_t)k * 32] = (uint32_t)chain_at(&im, k * LSTEP, &im.ctab[(size_t)k * 32 + 1]);
 	}
 	if (!(flags & SGI_BUILD_NO_FP64))
 	{
@@ -2632,6 +2949,7 @@ int upload_image(GridImage& im, int device, sgi_grid_t* out)
 	}
 	if (rc) { free_grid(d); return rc; }
 	d->nlch = im.nlch;
+	d->mean_active = im.mean_active;
 	d->skip_floor = d->skip_below = im.skip_floor;
 	d->f16_floor = im.f16_floor;
 	d->parent_h = std::move(im.parent_h);
@@ -2655,7 +2973,7 @@ int upload_image(GridImage& im, int device, sgi_grid_t* out)
 // written before it.  Native byte order: a cache is read back on the machine
 // (or an identical one) that wrote it.
 constexpr char CACHE_MAGIC[8] = { 'S', 'G', 'I', 'L', 'A', 'Y', 'O', 'T' };
-constexpr uint32_t CACHE_VERSION = 3;
+constexpr uint32_t CACHE_VERSION = 4;
 
 struct CacheKey
 {
@@ -2753,6 +3071,7 @@ void cache_fields(IO& io, Image& im)
 {
 	io.val(im.dim); io.val(im.nno); io.val(im.TD); io.val(im.ld); io.val(im.nlch); io.val(im.skip_floor);
 	io.val(im.f16_floor);
+	io.val(im.mean_active);
 	auto& I = im.info;
 	io.val(I.dim); io.val(I.nno); io.val(I.TotalDof); io.val(I.ld); io.val(I.max_comps); io.val(I.tree_depth);
 	io.val(I.tree_roots); io.val(I.multi_delta); io.val(I.ncoarse); io.val(I.comps); io.val(I.device_bytes);
@@ -3049,32 +3368,79 @@ int group_clen(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng, con
 	                 : (chunk >= maxnno ? 0 : chunk);
 }
 
-// Scratch bytes of a launch group's hit lists when it runs the two-phase
-// small-batch kernels (FP64, or FP32C on grids that keep their FP64 rows; not
-// node-chunked; fewer points than resident warps; lists within
-// LIST_SCRATCH_MAX), else 0.
-constexpr size_t LIST_SCRATCH_MAX = 256ull << 20;
+// How a launch group's points run in two phases.
+struct ListPlan
+{
+	int clen = 0;            // nodes per phase-1 chunk
+	long long items = 0;     // (point, chunk) items
+	long long cap = 0;       // list entries
+	bool pooled = false;     // entries come from a common pool, not one per (point, node)
+	size_t bytes = 0;        // scratch; 0: the group runs the one-phase kernels
+};
 
-size_t list_scratch(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng, const long long* pt_offsets,
+// A batch runs in two phases when it is not node-chunked and, on grids that
+// keep their FP64 rows, holds fewer points than the GPU does warps; FP64 also
+// up to four points per mean active node, at most LIST_POINTS.  Beyond that,
+// one warp per point wins: its time is the longest point's chain (several
+// times the mean; 1,500 to 3,000 points of a 150,000-node d=59 grid, 118
+// outputs, 0.97 ms, 6,000 points 1.18 ms, against 0.36, 0.55 and 0.88 in two
+// phases; on a 60,000-node d=30 grid of 64 outputs, half the active nodes,
+// 0.26 ms up to 3,000 points, against 0.23 at 1,500 and 0.34 at 3,000), then
+// its throughput, and two phases move the lists through memory.
+// Lists that would hold one entry per (point, node) within LIST_DIRECT bytes
+// do; others share a pool of four times the entries that the grids' mean
+// active counts predict for uniform points, at most LIST_SCRATCH_MAX bytes.
+constexpr size_t LIST_DIRECT = 24ull << 20;
+constexpr size_t LIST_SCRATCH_MAX = 256ull << 20;
+constexpr double LIST_POINTS = 8192.0;
+// Phase 2 by blocks while there are at most this many (point, 32 outputs) per
+// SM: 75 points of 570 hits, 118 outputs, take 25 us against 88 by warps; six
+// waves of blocks take about what the warps' longest point does.
+constexpr long long STAGE_ITEMS_PER_SM = 12;
+
+ListPlan list_plan(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng, const long long* pt_offsets,
 	int precision, int clen)
 {
+	ListPlan P;
 	const long long np = pt_offsets[gb + ng] - pt_offsets[gb];
-	if ((precision != SGI_FP64 && precision != SGI_FP32C) || clen || np == 0 || np >= (long long)W->sms * WARPS)
-		return 0;
-	long long items = 0;
+	if ((precision != SGI_FP64 && precision != SGI_FP32C) || clen || np == 0) return P;
+	double nodes = 0.0, active = 0.0;
+	int maxnno = 0;
 	for (int k = 0; k < ng; k++)
 	{
-		if (!grids[gb + k]->s64) return 0;
-		items += (pt_offsets[gb + k + 1] - pt_offsets[gb + k]) * grids[gb + k]->nlch;
+		const long long n = pt_offsets[gb + k + 1] - pt_offsets[gb + k];
+		if (!grids[gb + k]->s64) return P;
+		nodes += (double)n * grids[gb + k]->nno;
+		active += (double)n * grids[gb + k]->mean_active;
+		if (n) maxnno = std::max(maxnno, grids[gb + k]->nno);
 	}
-	if (items == 0) return 0;
-	const size_t bytes = (((size_t)items * 4 + 255) & ~(size_t)255) + (size_t)items * LCS * 12;
-	return bytes <= LIST_SCRATCH_MAX ? bytes : 0;
+	if (maxnno == 0) return P;
+	const double most = precision == SGI_FP64 ? std::min(LIST_POINTS, 4.0 * active / (double)np) : 0.0;
+	if (np >= (long long)W->sms * WARPS && (double)np > most) return P;
+	// about 96 items per SM, twice the warps it holds, but chunks no shorter
+	// than the chain table's step, and with no more than 16 hits expected (an
+	// item of a long point with a few hundred outlasts the others: 1,500 points
+	// of a 150,000-node grid, walk 310 us at 32,768 nodes a chunk, 134 at 4,096,
+	// 143 at 2,048, where every item's start-up shows)
+	long long c = LSTEP;
+	while (c < maxnno && nodes / (double)c > 96.0 * W->sms && active / nodes * (double)c <= 16.0) c *= 2;
+	P.clen = (int)c;
+	for (int k = 0; k < ng; k++)
+		P.items += (pt_offsets[gb + k + 1] - pt_offsets[gb + k]) * ((grids[gb + k]->nno + c - 1) / c);
+	const long long all = P.items * c;
+	P.pooled = all * 12 > (long long)LIST_DIRECT;
+	const long long most_entries = (long long)(LIST_SCRATCH_MAX - 256 - ((size_t)P.items * 8 + 255)) / 12;
+	P.cap = !P.pooled ? all : (long long)std::min({ nodes, std::max(4.0 * active, 1048576.0), (double)most_entries });
+	// a pool that may not hold what is expected is not worth its walk
+	if (P.cap <= 0 || (P.pooled && active > 0.75 * (double)P.cap)) return ListPlan{};
+	P.bytes = 256 + (((size_t)P.items * 8 + 255) & ~(size_t)255) + (size_t)P.cap * 12;
+	return P;
 }
 
-// The two launches of a two-phase group; buf holds list_scratch() bytes.
-int launch_lists(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng, const long long* pt_offsets,
-	const double* x, double* out, int precision, char* buf, cudaStream_t stream, int* phase2_blocks)
+// The two launches of a two-phase group; buf holds P.bytes bytes.
+int launch_lists(const DeviceWork* W, const ListPlan& P, const sgi_grid_t* grids, int gb, int ng,
+	const long long* pt_offsets, const double* x, double* out, int precision, char* buf, cudaStream_t stream,
+	int* phase2_blocks, int* phase2_threads)
 {
 	const sgi_grid* g0 = grids[0];
 	const long long p0 = pt_offsets[gb];
@@ -3086,33 +3452,64 @@ int launch_lists(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng, c
 		const sgi_grid* g = grids[gb + k];
 		la.g[k] = desc_of(g, pt_offsets[gb + k] - p0, precision);
 		la.ctab[k] = g->ctab;
-		la.nch[k] = g->nlch;
+		la.nch[k] = (g->nno + P.clen - 1) / P.clen;
 		la.ibeg[k] = items;
-		items += (pt_offsets[gb + k + 1] - pt_offsets[gb + k]) * g->nlch;
+		items += (pt_offsets[gb + k + 1] - pt_offsets[gb + k]) * la.nch[k];
 	}
 	la.ibeg[ng] = items;
 	la.x = x + (size_t)p0 * g0->dim;
 	la.out = out + (size_t)p0 * g0->TD;
 	la.npts = pt_offsets[gb + ng] - p0;
 	la.ngrids = ng; la.dim = g0->dim; la.TD = g0->TD;
-	la.hcnt = reinterpret_cast<uint32_t*>(buf);
-	la.hnode = reinterpret_cast<uint32_t*>(buf + (((size_t)items * 4 + 255) & ~(size_t)255));
-	la.hw = reinterpret_cast<double*>(la.hnode + (size_t)items * LCS);
-	const size_t sm1 = (size_t)WARPS * g0->dim * sizeof(double);
+	la.clen = P.clen;
+	la.cap = P.cap;
+	la.cursor = P.pooled ? reinterpret_cast<unsigned long long*>(buf) : nullptr;
+	la.item = reinterpret_cast<uint2*>(buf + 256);
+	la.hw = reinterpret_cast<double*>(buf + 256 + (((size_t)items * 8 + 255) & ~(size_t)255));
+	la.hnode = reinterpret_cast<uint32_t*>(la.hw + P.cap);
+	const int ncb = (g0->TD + 31) / 32;
+	const bool stage = la.npts * ncb <= STAGE_ITEMS_PER_SM * W->sms;
+	la.prefetch = stage;
+	const size_t sm1 = (size_t)WARPS * walk_stride(g0->dim) * sizeof(double);
+	if (sm1 > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(walk_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
 	int b1 = 0;
 	int rc = occupancy_grid(walk_chunks_kernel, sm1, W->sms, &b1);
 	if (rc) return rc;
+	const long long warps1 = (long long)b1 * WARPS;
 	b1 = (int)std::min<long long>(b1, (items + WARPS - 1) / WARPS);
+	// work beyond one item per warp is handed out by counters
+	const bool queued = items > warps1 || la.npts * ncb > 8ll * W->sms;
+	if (queued) la.counter = reinterpret_cast<unsigned long long*>(buf) + 1;
+	if (P.pooled || queued) CUDA_TRY(cudaMemsetAsync(buf, 0, 3 * sizeof(unsigned long long), stream));
 	walk_chunks_kernel<<<b1, BLOCK, sm1, stream>>>(la);
 	CUDA_TRY(cudaGetLastError());
-	const size_t sm2 = (size_t)(LBLOCK / 32) * list_stride() * sizeof(double);
-	CUDA_TRY(cudaFuncSetAttribute(fwd_f64_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
 	int b2 = 0;
-	rc = occupancy_grid(fwd_f64_list_kernel, sm2, W->sms, &b2, LBLOCK);
-	if (rc) return rc;
-	const long long items2 = la.npts * ((g0->TD + 31) / 32);
-	b2 = (int)std::min<long long>(b2, (items2 + LBLOCK / 32 - 1) / (LBLOCK / 32));
-	fwd_f64_list_kernel<<<b2, LBLOCK, sm2, stream>>>(la);
+	// (point, 32 outputs) blocks for a few waves of them; beyond, warps
+	if (stage)
+	{
+		constexpr int NC = 1, NP = 3, SROWS = 64, SRING = 4, SENTRIES = 2048;
+		void (*k2)(ListArgs) = fwd_f64_stage_kernel<NC, NP, SROWS, SRING, SENTRIES>;
+		const size_t sm2 = stage_smem<NC, SROWS, SRING, SENTRIES>();
+		CUDA_TRY(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
+		*phase2_threads = (NC + NP) * 32;
+		rc = occupancy_grid(k2, sm2, W->sms, &b2, *phase2_threads);
+		if (rc) return rc;
+		b2 = (int)std::min<long long>(b2, la.npts * ncb);
+		k2<<<b2, *phase2_threads, sm2, stream>>>(la);
+	}
+	else
+	{
+		const bool wide = g0->ld > 32;
+		void (*k2)(ListArgs) = wide ? fwd_f64_gather_kernel<2, 16> : fwd_f64_gather_kernel<1, 32>;
+		const size_t sm2 = (size_t)WARPS * cols_stride(g0->dim) * sizeof(double);
+		if (sm2 > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
+		rc = occupancy_grid(k2, sm2, W->sms, &b2);
+		if (rc) return rc;
+		const long long items2 = la.npts * (wide ? (g0->TD + 63) / 64 : ncb);
+		b2 = (int)std::min<long long>(b2, (items2 + WARPS - 1) / WARPS);
+		k2<<<b2, BLOCK, sm2, stream>>>(la);
+		*phase2_threads = BLOCK;
+	}
 	CUDA_TRY(cudaGetLastError());
 	*phase2_blocks = b2;
 	return SGI_OK;
@@ -3152,8 +3549,8 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 	for (int gb = 0; gb < ngrids; gb += MAXG)
 	{
 		const int ng = std::min(MAXG, ngrids - gb);
-		lneed = std::max(lneed, list_scratch(W, grids, gb, ng, pt_offsets, precision,
-		                                     group_clen(W, grids, gb, ng, pt_offsets, precision, chunk)));
+		lneed = std::max(lneed, list_plan(W, grids, gb, ng, pt_offsets, precision,
+		                                  group_clen(W, grids, gb, ng, pt_offsets, precision, chunk)).bytes);
 	}
 	PoolScratch pooled;
 	char* lbuf = nullptr;
@@ -3189,15 +3586,16 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 		if (lbuf)
 		{
 			const int gclen = group_clen(W, grids, gb, ng, pt_offsets, precision, chunk);
-			if (list_scratch(W, grids, gb, ng, pt_offsets, precision, gclen))
+			const ListPlan P = list_plan(W, grids, gb, ng, pt_offsets, precision, gclen);
+			if (P.bytes)
 			{
-				int b2 = 0;
-				rc = launch_lists(W, grids, gb, ng, pt_offsets, x, out, precision, lbuf, stream, &b2);
+				int b2 = 0, t2 = 0;
+				rc = launch_lists(W, P, grids, gb, ng, pt_offsets, x, out, precision, lbuf, stream, &b2, &t2);
 				if (rc) return rc;
 				launches += 2;
 				g_stats.kernels += 2;
 				g_stats.grid_blocks = b2;
-				g_stats.block_threads = LBLOCK;
+				g_stats.block_threads = t2;
 				g_stats.points += p1 - p0;
 				continue;
 			}
@@ -3267,7 +3665,7 @@ int count_launches(const DeviceWork* W, int ngrids, const sgi_grid_t* grids, con
 		int maxnno = 0;
 		for (int k = 0; k < ng; k++) maxnno = std::max(maxnno, grids[gb + k]->nno);
 		const int clen = chunk >= maxnno ? 0 : chunk;
-		const size_t lb = list_scratch(W, grids, gb, ng, pt_offsets, precision, clen);
+		const size_t lb = list_plan(W, grids, gb, ng, pt_offsets, precision, clen).bytes;
 		*list_bytes = std::max(*list_bytes, lb);
 		n += lb ? 2 : passes * (clen ? (maxnno + clen - 1) / clen : 1);
 	}
