@@ -865,11 +865,24 @@ __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32c_kernel(const __grid_cons
 // about 40 ranges.
 constexpr int SCAP = 96;
 
+// Big terms listed (16-byte entries) by the kernels of up to LISTB_MAX outputs
+// per lane: groups are taken whole at every step, so that at most a group's
+// remainder is left when a step adds up to 32.  With eight outputs per lane
+// the registers hold two FP64 rows either way, and the list only takes L1
+// from re-read rows (131,072 points, 256 outputs: 5.95 ms with it, 5.41
+// without; 118 outputs: 4.79 with, 5.31 without; 64: 1.83 and 1.98; 32: 1.54
+// and 1.77).
+constexpr int BCAP = 40;
+constexpr int LISTB_MAX = 4;
+
 // Shared memory per warp of the descent form, in doubles: the stack (SCAP
 // 16-byte entries), the fine-term list (whose first 32 doubles hold the chain
 // weights at a chunk start, before any term is listed), the list of fine
-// terms read from FP16 rows, and the point.
-__host__ __device__ __forceinline__ int desc_stride(int dim) { return 2 * SCAP + 2 * FCAP + ((dim + 1) & ~1); }
+// terms read from FP16 rows, that of big terms, and the point.
+__host__ __device__ __forceinline__ int desc_stride(int dim, bool listb)
+{
+	return 2 * SCAP + 2 * FCAP + (listb ? 2 * BCAP : 0) + ((dim + 1) & ~1);
+}
 
 // FP16 rows: row n holds its surpluses times 2^k_n as IEEE half precision,
 // k_n = 14 - floor(log2(rowmax_n)), so that the row's largest magnitude lies
@@ -897,19 +910,29 @@ __device__ __forceinline__ uint4 pack_seg(uint32_t b, uint32_t e, double w)
 	return make_uint4(b, e, (uint32_t)__double2loint(w), (uint32_t)__double2hiint(w));
 }
 
-template <int V, int E, int Q, int MINB, bool FULLROW>
+// QV: fine rows per group at eight outputs per lane; narrower rows take more,
+// up to FLUSH, so that a lane's loads in flight fill as many registers.
+template <int V, int E, int QV, int MINB, bool FULLROW>
 __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32d_kernel(const __grid_constant__ FwdArgs a)
 {
+	constexpr int Q = QV * 8 / (V * E) < FLUSH ? QV * 8 / (V * E) : FLUSH;
+	// big rows per group: 32 registers of loads in flight, 64 in the variant
+	// of fewer warps
+	constexpr int QB0 = (MINB == 2 ? 32 : 16) / (V * E);
+	constexpr int QB = QB0 < 8 ? QB0 : 8;
+	constexpr bool LISTB = V * E <= LISTB_MAX;
+	static_assert(QB >= 2 && 31 + QB <= BCAP, "the big-term list holds a remainder and a step's hits");
 	static_assert(FLUSH % Q == 0 || Q % FLUSH == 0, "groups of Q must tile the flush interval");
 	static_assert(32 % Q == 0, "groups of Q must tile a step's hits");
 	extern __shared__ double smem[];
 	const int lane = threadIdx.x & 31;
-	double* wbase = smem + (threadIdx.x >> 5) * desc_stride(a.dim);
+	double* wbase = smem + (threadIdx.x >> 5) * desc_stride(a.dim, LISTB);
 	uint4* stk = reinterpret_cast<uint4*>(wbase);
 	uint2* fl = reinterpret_cast<uint2*>(wbase + 2 * SCAP);
 	double* wchain = wbase + 2 * SCAP;     // aliases fl: used before any term is listed
 	uint2* fl16 = reinterpret_cast<uint2*>(wbase + 2 * SCAP + FCAP);
-	double* xs = wbase + 2 * SCAP + 2 * FCAP;
+	uint4* fb = reinterpret_cast<uint4*>(wbase + 2 * SCAP + 2 * FCAP);   // {FP64 copy row, -, weight}
+	double* xs = wbase + 2 * SCAP + 2 * FCAP + (LISTB ? 2 * BCAP : 0);
 	// FP16 rows serve launches whose lanes own two blocks of four outputs of
 	// full 256-output passes (the layout of the rows)
 	constexpr bool F16 = V == 2 && E == 4 && FULLROW;
@@ -980,7 +1003,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32d_kernel(const __grid_cons
 			for (int v = 0; v < V; v++)
 #pragma unroll
 				for (int e = 0; e < E; e++) part[v][e] = 0.f;
-			int cnt = 0, cnt16 = 0, since = 0;
+			int cnt = 0, cnt16 = 0, cntb = 0, since = 0;
 			auto flush = [&]()
 			{
 #pragma unroll
@@ -1087,6 +1110,31 @@ __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32d_kernel(const __grid_cons
 					if (since >= FLUSH) { flush(); since = 0; }
 				}
 			};
+			// big-term list entries [h, hend), N at a time
+			auto bigs = [&](auto n, int h, int hend)
+			{
+				constexpr int N = decltype(n)::value;
+				for (; h + N <= hend; h += N)
+				{
+					double sv[N][V][E], wq[N];
+#pragma unroll
+					for (int q = 0; q < N; q++)
+					{
+						const uint4 t = fb[h + q];
+						wq[q] = __hiloint2double((int)t.w, (int)t.z);
+						const double* row = s64l + (size_t)t.x * ld;
+#pragma unroll
+						for (int v = 0; v < V; v++)
+							load_row<E>(row, v * 32 * E, FULLROW || lcol + v * 32 * E < (int)ld, sv[q][v]);
+					}
+#pragma unroll
+					for (int q = 0; q < N; q++)
+#pragma unroll
+						for (int v = 0; v < V; v++)
+#pragma unroll
+							for (int e = 0; e < E; e++) acc[v][e] = fma(wq[q], sv[q][v][e], acc[v][e]);
+				}
+			};
 			while (size > 0)
 			{
 				const int B = max(1, min(32, room - size));
@@ -1163,7 +1211,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32d_kernel(const __grid_cons
 				const bool big = hit && ni.w != DESC_NONE && bound >= big_below;
 				const bool fine = hit && !big && bound >= skip_below;
 				const bool half = fine && bound < f16_below;
-				unsigned cm = __ballot_sync(FULL, big);
+				const unsigned cm = __ballot_sync(FULL, big);
 				const unsigned fm = __ballot_sync(FULL, fine && !half);
 				const unsigned hm = __ballot_sync(FULL, half);
 				const unsigned below = (1u << lane) - 1u;
@@ -1171,33 +1219,58 @@ __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32d_kernel(const __grid_cons
 				if (half) fl16[cnt16 + __popc(hm & below)] = make_uint2(c, __float_as_uint(f16_weight(wf, ni.z)));
 				cnt += __popc(fm);
 				cnt16 += __popc(hm);
-				while (cm)
+				if constexpr (LISTB)
 				{
-					const int k0 = __ffs(cm) - 1;
-					cm &= cm - 1;
-					const bool two = cm != 0u;
-					const int k1 = two ? __ffs(cm) - 1 : k0;
-					if (two) cm &= cm - 1;
-					const double w0 = __shfl_sync(FULL, w, k0);
-					const double w1 = __shfl_sync(FULL, w, k1);
-					const double* row0 = s64l + (size_t)__shfl_sync(FULL, ni.w, k0) * ld;
-					const double* row1 = s64l + (size_t)__shfl_sync(FULL, ni.w, k1) * ld;
-					double s0[V][E], s1[V][E];
-#pragma unroll
-					for (int v = 0; v < V; v++)
+					if (cm)
 					{
-						const bool in = FULLROW || lcol + v * 32 * E < (int)ld;
-						load_row<E>(row0, v * 32 * E, in, s0[v]);
-						load_row<E>(row1, v * 32 * E, in && two, s1[v]);
-					}
-#pragma unroll
-					for (int v = 0; v < V; v++)
-#pragma unroll
-						for (int e2 = 0; e2 < E; e2++)
+						if (big) fb[cntb + __popc(cm & below)] = pack_seg(ni.w, 0u, w);
+						cntb += __popc(cm);
+						const int wholeb = cntb - cntb % QB;
+						if (wholeb)
 						{
-							acc[v][e2] = fma(w0, s0[v][e2], acc[v][e2]);
-							if (two) acc[v][e2] = fma(w1, s1[v][e2], acc[v][e2]);
+							// all whole groups; the remainder (< QB entries) moves to the front
+							__syncwarp();
+							bigs(std::integral_constant<int, QB>(), 0, wholeb);
+							const int rem = cntb - wholeb;
+							uint4 t = make_uint4(0u, 0u, 0u, 0u);
+							if (lane < rem) t = fb[wholeb + lane];
+							__syncwarp();
+							if (lane < rem) fb[lane] = t;
+							cntb = rem;
 						}
+					}
+				}
+				else
+				{
+					// two at a time (two FP64 rows in flight)
+					for (unsigned c2 = cm; c2;)
+					{
+						const int k0 = __ffs(c2) - 1;
+						c2 &= c2 - 1;
+						const bool two = c2 != 0u;
+						const int k1 = two ? __ffs(c2) - 1 : k0;
+						if (two) c2 &= c2 - 1;
+						const double w0 = __shfl_sync(FULL, w, k0);
+						const double w1 = __shfl_sync(FULL, w, k1);
+						const double* row0 = s64l + (size_t)__shfl_sync(FULL, ni.w, k0) * ld;
+						const double* row1 = s64l + (size_t)__shfl_sync(FULL, ni.w, k1) * ld;
+						double s0[V][E], s1[V][E];
+#pragma unroll
+						for (int v = 0; v < V; v++)
+						{
+							const bool in = FULLROW || lcol + v * 32 * E < (int)ld;
+							load_row<E>(row0, v * 32 * E, in, s0[v]);
+							load_row<E>(row1, v * 32 * E, in && two, s1[v]);
+						}
+#pragma unroll
+						for (int v = 0; v < V; v++)
+#pragma unroll
+							for (int e2 = 0; e2 < E; e2++)
+							{
+								acc[v][e2] = fma(w0, s0[v][e2], acc[v][e2]);
+								if (two) acc[v][e2] = fma(w1, s1[v][e2], acc[v][e2]);
+							}
+					}
 				}
 				if (cnt >= 32)
 				{
@@ -1226,6 +1299,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32d_kernel(const __grid_cons
 					__syncwarp();
 					cnt16 = rem;
 				}
+			}
+			if (cntb)
+			{
+				__syncwarp();
+				bigs(std::integral_constant<int, 1>(), 0, cntb);
 			}
 			if (cnt)
 			{
@@ -2512,15 +2590,25 @@ int chunk_rows_env() { return g_chunk_override.load(); }
 // SGI_FP32C_VARIANT at start-up) fixed.
 std::atomic<int> g_variant{[]() { const char* e = getenv("SGI_FP32C_VARIANT"); return e ? atoi(e) : -1; }()};
 
-// The automatic FP32C variant: eight fine rows in flight per warp (2) for a
-// batch of fewer than 64 points per SM, whose warps wait on their rows (on a
-// 200k-node d=59 grid, 16 / 1,024 / 8,192 points: 242 / 451 / 994 us against
-// 327 / 661 / 1,130 us for variant 1), else two rows at 4 blocks per SM (1),
-// the faster at a million points.
-int auto_variant(int variant, long long npts, int sms)
+// Outputs per lane of a pass of `cols` columns over rows of stride ld.
+int lane_outputs(int ld, int cols) { return ld <= 32 ? 1 : cols <= 64 ? 2 : cols <= 128 ? 4 : 8; }
+
+// The automatic FP32C variant.  A small batch waits on its rows, with few
+// points per warp slot: more rows in flight per warp (2, then 0) beat more
+// warps (1) up to a number of points per SM that falls with the row width,
+// as a narrow row's adds hide less (d=59 and d=30 grids of 60,000 to 150,000
+// nodes; us for variants 0 / 1 / 2.  256 outputs: 10,007 points 624 / 747 /
+// 576, 20,000 990 / 1,104 / 986, 40,000 1,792 / 1,772 / 1,821.  118 outputs:
+// 5,000 491 / 609 / 444, 10,007 573 / 641 / 603, 20,000 912 / 968 / 976,
+// 40,000 1,627 / 1,568 / 1,780.  64 outputs: 2,000 155 / 157 / 146, 5,000
+// 174 / 173 / 194).
+int auto_variant(int variant, long long npts, int sms, int outputs)
 {
 	if (variant >= 0) return variant;
-	return npts < (long long)sms * 64 ? 2 : 1;
+	const long long per_sm = npts / sms;
+	if (outputs == 8) return per_sm < 128 ? 2 : 1;
+	if (outputs == 4) return per_sm < 48 ? 2 : per_sm < 256 ? 0 : 1;
+	return per_sm < 16 ? 2 : 1;
 }
 
 uint32_t float_bits(float f)
@@ -2583,10 +2671,10 @@ void (*select_fwd(int precision, int ld, int cols, int variant = 0, bool descent
 }
 
 // Dynamic shared memory of a forward launch.
-size_t fwd_smem(int precision, int dim, bool descent = false)
+size_t fwd_smem(int precision, int dim, bool descent = false, int outputs = 8)
 {
 	if (precision != SGI_FP32C) return (size_t)WARPS * hit_stride(dim) * sizeof(double);
-	return (size_t)WARPS * (descent ? desc_stride(dim) : list_stride(dim)) * sizeof(double);
+	return (size_t)WARPS * (descent ? desc_stride(dim, outputs <= LISTB_MAX) : list_stride(dim)) * sizeof(double);
 }
 
 template <int R>
@@ -3615,8 +3703,6 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 		const bool small = a.npts < (long long)W->sms * WARPS;
 		// small unchunked FP64 batches: one warp per (point, 32 outputs)
 		const bool cols_mode = precision == SGI_FP64 && small && clen == 0;
-		const size_t smem = cols_mode ? (size_t)WARPS * cols_stride(g0->dim) * sizeof(double)
-		                              : fwd_smem(precision, g0->dim, descent);
 		for (int ob = 0; ob < g0->TD; ob += PASS)
 		for (int c = 0; c < std::max(nchunks, 1); c++)
 		{
@@ -3627,8 +3713,11 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 			a.counter = counters ? counters + launches : W->counters + (W->next.fetch_add(1) % NCOUNTERS);
 			CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream));
 			const int cols = std::min(g0->TD - ob, PASS);
+			const int outputs = lane_outputs(g0->ld, cols);
+			const size_t smem = cols_mode ? (size_t)WARPS * cols_stride(g0->dim) * sizeof(double)
+			                              : fwd_smem(precision, g0->dim, descent, outputs);
 			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel
-				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, W->sms), descent);
+				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, W->sms, outputs), descent);
 			if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 			int blocks = 0;
 			rc = occupancy_grid(kern, smem, W->sms, &blocks);
@@ -4055,16 +4144,17 @@ extern "C" int sgi_interpolate_noalloc(int ngrids, const sgi_grid_t* grids, cons
 		const bool descent = precision == SGI_FP32C && descent_ok(grids, gb, ng, false);
 		const bool small = a.npts < (long long)sms * WARPS;
 		const bool cols_mode = precision == SGI_FP64 && small;
-		const size_t smem = cols_mode ? (size_t)WARPS * cols_stride(g0->dim) * sizeof(double)
-		                              : fwd_smem(precision, g0->dim, descent);
 		for (int ob = 0; ob < g0->TD; ob += PASS)
 		{
 			a.o_begin = ob;
 			a.counter = counters + slot++;
 			CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream));
 			const int cols = std::min(g0->TD - ob, PASS);
+			const int outputs = lane_outputs(g0->ld, cols);
+			const size_t smem = cols_mode ? (size_t)WARPS * cols_stride(g0->dim) * sizeof(double)
+			                              : fwd_smem(precision, g0->dim, descent, outputs);
 			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel
-				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, sms), descent);
+				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, sms, outputs), descent);
 			if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 			int blocks = 0;
 			rc = occupancy_grid(kern, smem, sms, &blocks);

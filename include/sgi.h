@@ -324,8 +324,10 @@ int sgi_set_chunk_rows(int rows);
  * order the FP64 additions of big terms and of FP32 partial sums differently,
  * so their results may differ in the last bits (all within the FP32C
  * tolerance).  variant < 0 or SGI_FP32C_AUTO restores the default,
- * automatic: 2 for a launch with fewer than 64 points per SM (9,472 on a
- * B200), else 1.  Returns the previous setting
+ * automatic by the points per SM and the width of a launch's rows: above 128
+ * outputs 2 for fewer than 128 points per SM (18,944 on a B200), else 1; above
+ * 64 outputs 2 for fewer than 48, 0 for fewer than 256, else 1; below, 2 for
+ * fewer than 16, else 1.  Returns the previous setting
  * (SGI_FP32C_AUTO for automatic), or a negative error code.  No reference
  * counterpart. */
 #define SGI_FP32C_AUTO 255
