@@ -1485,6 +1485,7 @@ struct ListArgs
 	int ngrids, dim, TD;
 	int clen;                    // nodes per chunk
 	int prefetch;                // bring listed rows into the L2
+	int any;                     // walk points with a non-finite coordinate too
 };
 static_assert(sizeof(ListArgs) <= 32764, "ListArgs exceeds the kernel parameter limit");
 
@@ -1538,7 +1539,7 @@ __global__ void __launch_bounds__(BLOCK, 5) walk_chunks_kernel(const __grid_cons
 		}
 		__syncwarp();
 		uint2 res = make_uint2(0u, HIT_BAD);
-		if (__all_sync(FULL, finite))
+		if (__all_sync(FULL, finite) || a.any)
 		{
 			const int len = (int)__shfl_sync(FULL, chain, 0);
 			// lane d >= 1 asks for the chain node at depth d, the word it holds
@@ -2157,11 +2158,19 @@ __device__ __forceinline__ double rcp_hat(double h)
 	return fma(r, fma(-h, r, 1.0), r);
 }
 
+// Warps that can share a point's dL/dx, and the most walk chunks they find its
+// hits in.
+constexpr int DXW = 4;
+constexpr int DX_ITEMS = 1024;
+
 // dL/dx terms of m <= 32 pairs of one point (lane k holds pair k's component
 // range and cs * w): each half-warp takes every other pair, a component per
 // lane (a node of a d=59 grid has ten on average), and adds to its own copy of
 // the point's gradient (gxs, gxs + dim), so that two pairs sharing a dimension
-// never meet.  dw/dx as w * slope / hat needs no products of the other hats;
+// never meet.  A point's pairs are taken in lists of 32; list l adds to copies
+// 2 (l mod DXW) and the next, so that DXW warps can share a point, and every
+// kernel adds the copies in the same order: dL/dx does not depend on which one
+// ran.  dw/dx as w * slope / hat needs no products of the other hats;
 // eight pairs' components are in flight while eight are added (with two, the
 // loads were what it waited on: 2.6 ms against 2.2 over 44M pairs).
 __device__ __forceinline__ void dx_pass(const GridDesc& G, const double* xs, double* gxs, int dim, uint32_t cptr,
@@ -2217,7 +2226,35 @@ __device__ __forceinline__ void dx_pass(const GridDesc& G, const double* xs, dou
 	}
 }
 
-__host__ __device__ __forceinline__ int bwd_stride(int dim) { return HCAP * 2 + 3 * dim + (dim & 1); }
+// A point's dL/dx from its copies.
+__device__ __forceinline__ double dx_sum(const double* gxs, int dim, int k)
+{
+	double t = gxs[k];
+#pragma unroll
+	for (int c = 1; c < 2 * DXW; c++) t += gxs[c * dim + k];
+	return t;
+}
+
+__host__ __device__ __forceinline__ int bwd_stride(int dim)
+{
+	return HCAP * 2 + (1 + 2 * DXW) * dim + (((1 + 2 * DXW) * dim) & 1);
+}
+
+// One point's dL/dx copies, walked by one warp.
+template <int R>
+__device__ __forceinline__ void point_dx(const GridDesc& G, const double* xs, double* gxs, Hit* hits, int dim,
+	const double* g, int lane)
+{
+	int l = 0;
+	walk_lists(G, xs, hits, lane, 0, G.nno, 1u, 0, [&](int m)
+	{
+		const Hit h = hits[min(lane, m - 1)];
+		const double w = lane < m ? node_weight(G, xs, hit_cptr(h), hit_ncomp(h)) : 0.0;
+		const double cs = rows_dot<R>(G.s64, (uint32_t)G.ld, h.node, m, lane, g);
+		dx_pass(G, xs, gxs + 2 * l * dim, dim, hit_cptr(h), hit_ncomp(h), cs * w, m, lane);
+		l = (l + 1) & (DXW - 1);
+	});
+}
 
 // dL/dx without dL/dsurplus: one warp per point, 32 hits at a time.
 template <int R>
@@ -2229,27 +2266,134 @@ __global__ void __launch_bounds__(BLOCK, R == 8 ? 2 : 3) bwd_points_kernel(const
 	Hit* hits = reinterpret_cast<Hit*>(wbase);
 	double* xs = wbase + 2 * HCAP;
 	double* gxs = xs + a.dim;
-	const GridDesc& G = a.G;
 	for (;;)
 	{
 		long long p = 0;
 		if (lane == 0) p = (long long)atomicAdd(a.counter, 1ull);
 		p = __shfl_sync(FULL, p, 0);
 		if (p >= a.npts) break;
-		for (int k = lane; k < a.dim; k += 32) { xs[k] = a.x[(size_t)p * a.dim + k]; gxs[k] = 0.0; gxs[a.dim + k] = 0.0; }
+		for (int k = lane; k < a.dim; k += 32) xs[k] = a.x[(size_t)p * a.dim + k];
+		for (int k = lane; k < 2 * DXW * a.dim; k += 32) gxs[k] = 0.0;
 		double g[R];
 		bwd_row<R, false>(a.gout + (size_t)p * a.TD, a.TD, lane, g);
 		__syncwarp();
-		walk_lists(G, xs, hits, lane, 0, G.nno, 1u, 0, [&](int m)
+		point_dx<R>(a.G, xs, gxs, hits, a.dim, g, lane);
+		__syncwarp();
+		for (int k = lane; k < a.dim; k += 32) a.gx[(size_t)p * a.dim + k] = dx_sum(gxs, a.dim, k);
+		__syncwarp();
+	}
+}
+
+// The same for a batch that fits few waves of warps, whose time is the longest
+// point's (2,440 hits against 544 on average): the walk in parallel chunks
+// (walk_chunks_kernel), then DXW warps per point.  A point whose lists found
+// no room is walked by its first warp.
+template <int R>
+__global__ void __launch_bounds__(32 * DXW, R == 8 ? 4 : 6) bwd_points_list_kernel(const __grid_constant__ ListArgs a,
+	const double* __restrict__ gout, double* __restrict__ gx)
+{
+	extern __shared__ double smem[];
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	Hit* hits = reinterpret_cast<Hit*>(smem);
+	double* xs = smem + 2 * HCAP;
+	double* gxs = xs + a.dim;
+	uint32_t* ipre = reinterpret_cast<uint32_t*>(smem + bwd_stride(a.dim));
+	uint32_t* ioff = ipre + DX_ITEMS;
+	uint32_t* sums = ioff + DX_ITEMS;
+	const GridDesc& G = a.g[0];
+	const int nch = a.nch[0];
+	__shared__ long long next;
+	for (;;)
+	{
+		if (tid == 0) next = (long long)atomicAdd(a.counter + 1, 1ull);
+		__syncthreads();
+		const long long p = next;
+		if (p >= a.npts) break;
+		for (int k = tid; k < a.dim; k += 32 * DXW) xs[k] = a.x[(size_t)p * a.dim + k];
+		for (int k = tid; k < 2 * DXW * a.dim; k += 32 * DXW) gxs[k] = 0.0;
+		double g[R];
+		bwd_row<R, false>(gout + (size_t)p * a.TD, a.TD, lane, g);
+		// the point's items: entries and the hits before them
+		constexpr int IPT = DX_ITEMS / (32 * DXW);
+		uint2 v[IPT];
+		uint32_t mine = 0;
+		bool o = false;
+#pragma unroll
+		for (int j = 0; j < IPT; j++)
 		{
-			const Hit h = hits[min(lane, m - 1)];
-			const double w = lane < m ? node_weight(G, xs, hit_cptr(h), hit_ncomp(h)) : 0.0;
-			const double cs = rows_dot<R>(G.s64, (uint32_t)G.ld, h.node, m, lane, g);
-			dx_pass(G, xs, gxs, a.dim, hit_cptr(h), hit_ncomp(h), cs * w, m, lane);
-		});
-		__syncwarp();
-		for (int k = lane; k < a.dim; k += 32) a.gx[(size_t)p * a.dim + k] = gxs[k] + gxs[a.dim + k];
-		__syncwarp();
+			const int k = tid * IPT + j;
+			v[j] = k < nch ? __ldg(a.item + p * nch + k) : make_uint2(0u, 0u);
+			o = o || v[j].y == HIT_OVER;
+			mine += v[j].y;
+		}
+		const bool over = __syncthreads_or(o);
+		if (over)
+		{
+			if (warp == 0) point_dx<R>(G, xs, gxs, hits, a.dim, g, lane);
+		}
+		else
+		{
+			uint32_t incl = mine;
+#pragma unroll
+			for (int s = 1; s < 32; s <<= 1)
+			{
+				const uint32_t u = __shfl_up_sync(FULL, incl, s);
+				if (lane >= s) incl += u;
+			}
+			if (lane == 31) sums[warp] = incl;
+			__syncthreads();
+			uint32_t before = incl - mine, T = 0;
+#pragma unroll
+			for (int s = 0; s < DXW; s++)
+			{
+				if (s < warp) before += sums[s];
+				T += sums[s];
+			}
+#pragma unroll
+			for (int j = 0; j < IPT; j++)
+			{
+				ipre[tid * IPT + j] = before;
+				ioff[tid * IPT + j] = v[j].x;
+				before += v[j].y;
+			}
+			__syncthreads();
+			// this warp's next list: its entries, then their records, are loaded
+			// while the list before is taken
+			uint32_t node = 0u;
+			double w = 0.0;
+			auto entries = [&](uint32_t q)
+			{
+				const uint32_t h = q + (uint32_t)lane;
+				node = 0u;
+				w = 0.0;
+				if (h >= T) return;
+				// the item of hit h: the last with at most that many before it
+				int l = 0, e = nch;
+				while (e - l > 1)
+				{
+					const int c = (l + e) >> 1;
+					if (ipre[c] <= h) l = c;
+					else e = c;
+				}
+				const size_t at = (size_t)ioff[l] + (h - ipre[l]);
+				node = __ldg(a.hnode + at);
+				w = __ldg(a.hw + at);
+			};
+			entries(32 * warp);
+			for (uint32_t q = 32 * warp; q < T; q += 32 * DXW)
+			{
+				const int m = (int)min(T - q, 32u);
+				const uint32_t n0 = node;
+				const double w0 = w;
+				const uint4 r = lane < m ? __ldg(G.rec + n0) : make_uint4(0u, 0u, 0u, 0u);
+				if (q + 32 * DXW < T) entries(q + 32 * DXW);
+				const double cs = rows_dot<R>(G.s64, (uint32_t)G.ld, n0, m, lane, g);
+				dx_pass(G, xs, gxs + 2 * warp * a.dim, a.dim, r.y, r.z & 0xffu, cs * w0, m, lane);
+			}
+		}
+		__syncthreads();
+		for (int k = tid; k < a.dim; k += 32 * DXW) gx[(size_t)p * a.dim + k] = dx_sum(gxs, a.dim, k);
+		__syncthreads();
 	}
 }
 
@@ -2466,24 +2610,26 @@ __global__ void __launch_bounds__(BLOCK) bwd_join_kernel(const __grid_constant__
 	}
 }
 
-// dL/dx from the pairs' cs * w: one warp per point.
-__global__ void __launch_bounds__(BLOCK) bwd_dx_kernel(const __grid_constant__ BwdArgs a)
+// dL/dx from the pairs' cs * w: DXW warps per point.
+__global__ void __launch_bounds__(32 * DXW) bwd_dx_kernel(const __grid_constant__ BwdArgs a)
 {
 	extern __shared__ double smem[];
-	const int lane = threadIdx.x & 31;
-	double* xs = smem + (threadIdx.x >> 5) * 3 * a.dim;
+	__shared__ long long next;
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	double* xs = smem;
 	double* gxs = xs + a.dim;
 	const GridDesc& G = a.G;
 	for (;;)
 	{
-		long long p = 0;
-		if (lane == 0) p = (long long)atomicAdd(a.counter, 1ull);
-		p = __shfl_sync(FULL, p, 0);
+		if (tid == 0) next = (long long)atomicAdd(a.counter, 1ull);
+		__syncthreads();
+		const long long p = next;
 		if (p >= a.npts) break;
-		for (int k = lane; k < a.dim; k += 32) { xs[k] = a.x[(size_t)p * a.dim + k]; gxs[k] = 0.0; gxs[a.dim + k] = 0.0; }
-		__syncwarp();
+		for (int k = tid; k < a.dim; k += 32 * DXW) xs[k] = a.x[(size_t)p * a.dim + k];
+		for (int k = tid; k < 2 * DXW * a.dim; k += 32 * DXW) gxs[k] = 0.0;
+		__syncthreads();
 		const long long b = a.pair_off[p], e = a.pair_off[p + 1];
-		for (long long q = b; q < e; q += 32)
+		for (long long q = b + 32 * warp; q < e; q += 32 * DXW)
 		{
 			const int m = (int)min(32ll, e - q);
 			uint4 r = make_uint4(0u, 0u, 0u, 0u);
@@ -2493,11 +2639,10 @@ __global__ void __launch_bounds__(BLOCK) bwd_dx_kernel(const __grid_constant__ B
 				r = __ldg(G.rec + __ldg(a.pair_node + q + lane));
 				csw = a.pair_val[q + lane].w;
 			}
-			dx_pass(G, xs, gxs, a.dim, r.y, r.z & 0xffu, csw, m, lane);
+			dx_pass(G, xs, gxs + 2 * warp * a.dim, a.dim, r.y, r.z & 0xffu, csw, m, lane);
 		}
-		__syncwarp();
-		for (int k = lane; k < a.dim; k += 32) a.gx[(size_t)p * a.dim + k] = gxs[k] + gxs[a.dim + k];
-		__syncwarp();
+		__syncthreads();
+		for (int k = tid; k < a.dim; k += 32 * DXW) a.gx[(size_t)p * a.dim + k] = dx_sum(gxs, a.dim, k);
 	}
 }
 
@@ -2685,6 +2830,13 @@ void (*nodes_kernel(bool dot, bool vec))(BwdArgs)
 	if (R == 1) vec = false;   // one column per lane either way
 	return dot ? (vec ? bwd_nodes_kernel<R, true, R != 1> : bwd_nodes_kernel<R, true, false>)
 	           : (vec ? bwd_nodes_kernel<R, false, R != 1> : bwd_nodes_kernel<R, false, false>);
+}
+
+// Coordinates (FP32C: with its term lists) of the eight warps of a block past
+// 200 KB.
+bool dim_too_large(int precision, int dim)
+{
+	return (precision == SGI_FP32C ? fwd_smem(precision, dim, true) : (size_t)WARPS * dim * sizeof(double)) > 200 * 1024;
 }
 
 int pick_R(int cols)
@@ -3489,7 +3641,7 @@ constexpr double LIST_POINTS = 8192.0;
 constexpr long long STAGE_ITEMS_PER_SM = 12;
 
 ListPlan list_plan(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng, const long long* pt_offsets,
-	int precision, int clen)
+	int precision, int clen, double per_active = 4.0)
 {
 	ListPlan P;
 	const long long np = pt_offsets[gb + ng] - pt_offsets[gb];
@@ -3505,7 +3657,8 @@ ListPlan list_plan(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng,
 		if (n) maxnno = std::max(maxnno, grids[gb + k]->nno);
 	}
 	if (maxnno == 0) return P;
-	const double most = precision == SGI_FP64 ? std::min(LIST_POINTS, 4.0 * active / (double)np) : 0.0;
+	if ((size_t)WARPS * walk_stride(grids[gb]->dim) * sizeof(double) > 220 * 1024) return P;
+	const double most = precision == SGI_FP64 ? std::min(LIST_POINTS, per_active * active / (double)np) : 0.0;
 	if (np >= (long long)W->sms * WARPS && (double)np > most) return P;
 	// about 96 items per SM, twice the warps it holds, but chunks no shorter
 	// than the chain table's step, and with no more than 16 hits expected (an
@@ -3527,14 +3680,14 @@ ListPlan list_plan(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng,
 	return P;
 }
 
-// The two launches of a two-phase group; buf holds P.bytes bytes.
-int launch_lists(const DeviceWork* W, const ListPlan& P, const sgi_grid_t* grids, int gb, int ng,
+// Phase 1 of a two-phase group; buf holds P.bytes bytes.  Fills in `la` for
+// phase 2 (queued: phase 2 takes its items from a counter).
+int launch_walk(const DeviceWork* W, const ListPlan& P, const sgi_grid_t* grids, int gb, int ng,
 	const long long* pt_offsets, const double* x, double* out, int precision, char* buf, cudaStream_t stream,
-	int* phase2_blocks, int* phase2_threads)
+	bool prefetch, bool any, bool queued, ListArgs& la)
 {
-	const sgi_grid* g0 = grids[0];
+	const sgi_grid* g0 = grids[gb];
 	const long long p0 = pt_offsets[gb];
-	ListArgs la;
 	memset(&la, 0, sizeof(la));
 	long long items = 0;
 	for (int k = 0; k < ng; k++)
@@ -3557,22 +3710,36 @@ int launch_lists(const DeviceWork* W, const ListPlan& P, const sgi_grid_t* grids
 	la.item = reinterpret_cast<uint2*>(buf + 256);
 	la.hw = reinterpret_cast<double*>(buf + 256 + (((size_t)items * 8 + 255) & ~(size_t)255));
 	la.hnode = reinterpret_cast<uint32_t*>(la.hw + P.cap);
-	const int ncb = (g0->TD + 31) / 32;
-	const bool stage = la.npts * ncb <= STAGE_ITEMS_PER_SM * W->sms;
-	la.prefetch = stage;
+	la.prefetch = prefetch;
+	la.any = any;
 	const size_t sm1 = (size_t)WARPS * walk_stride(g0->dim) * sizeof(double);
 	if (sm1 > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(walk_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
 	int b1 = 0;
 	int rc = occupancy_grid(walk_chunks_kernel, sm1, W->sms, &b1);
 	if (rc) return rc;
-	const long long warps1 = (long long)b1 * WARPS;
-	b1 = (int)std::min<long long>(b1, (items + WARPS - 1) / WARPS);
 	// work beyond one item per warp is handed out by counters
-	const bool queued = items > warps1 || la.npts * ncb > 8ll * W->sms;
+	queued = queued || items > (long long)b1 * WARPS;
+	b1 = (int)std::min<long long>(b1, (items + WARPS - 1) / WARPS);
 	if (queued) la.counter = reinterpret_cast<unsigned long long*>(buf) + 1;
 	if (P.pooled || queued) CUDA_TRY(cudaMemsetAsync(buf, 0, 3 * sizeof(unsigned long long), stream));
 	walk_chunks_kernel<<<b1, BLOCK, sm1, stream>>>(la);
 	CUDA_TRY(cudaGetLastError());
+	return SGI_OK;
+}
+
+// The two launches of a two-phase group; buf holds P.bytes bytes.
+int launch_lists(const DeviceWork* W, const ListPlan& P, const sgi_grid_t* grids, int gb, int ng,
+	const long long* pt_offsets, const double* x, double* out, int precision, char* buf, cudaStream_t stream,
+	int* phase2_blocks, int* phase2_threads)
+{
+	const sgi_grid* g0 = grids[0];
+	const long long np = pt_offsets[gb + ng] - pt_offsets[gb];
+	const int ncb = (g0->TD + 31) / 32;
+	const bool stage = np * ncb <= STAGE_ITEMS_PER_SM * W->sms;
+	ListArgs la;
+	int rc = launch_walk(W, P, grids, gb, ng, pt_offsets, x, out, precision, buf, stream, stage, false,
+	                     np * ncb > 8ll * W->sms, la);
+	if (rc) return rc;
 	int b2 = 0;
 	// (point, 32 outputs) blocks for a few waves of them; beyond, warps
 	if (stage)
@@ -3633,7 +3800,7 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 	else return fail(SGI_E_INVALID, "unknown precision %d", precision);
 	// per warp: the point's coordinates, and for FP32C the term list and the
 	// weight stack (window walk) or the group-range stack (descent)
-	if (fwd_smem(precision, g0->dim, true) > 200 * 1024) return fail(SGI_E_RANGE, "dim %d too large for shared staging", g0->dim);
+	if (dim_too_large(precision, g0->dim)) return fail(SGI_E_RANGE, "dim %d too large for shared staging", g0->dim);
 	g_stats = sgi_launch_stats{};
 	size_t lneed = 0;
 	for (int gb = 0; gb < ngrids; gb += MAXG)
@@ -3940,6 +4107,53 @@ extern "C" int sgi_term_classes(sgi_grid_t g, long long npts, const double* x, l
 	return count_terms(g, npts, x, nullptr, out, stream);
 }
 
+namespace {
+
+// dL/dx alone in two phases when the stream is not being captured and the
+// scratch is there: batches of fewer points than the GPU holds warps, and up
+// to DX_LIST_PER_ACTIVE points per mean active node (a 50,000-node d=59 grid
+// of 118 outputs, 544 active nodes: 50 points 0.25 ms against 0.55 by one warp
+// per point, 500 0.30 / 0.55, 1,500 0.35 / 0.55, 3,000 0.53 / 0.62, 5,000
+// 0.74 / 0.68; the few points in flight at a time share fewer rows in the L2).
+constexpr double DX_LIST_PER_ACTIVE = 3.0;
+
+int backward_lists(DeviceWork* W, sgi_grid_t g, long long npts, const double* x, const double* gout, double* gx,
+	int R, cudaStream_t stream, bool* done)
+{
+	*done = false;
+	cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+	CUDA_TRY(cudaStreamIsCapturing(stream, &cap));
+	if (cap != cudaStreamCaptureStatusNone) return SGI_OK;
+	const long long offs[2] = { 0, npts };
+	const ListPlan P = list_plan(W, &g, 0, 1, offs, SGI_FP64, 0, DX_LIST_PER_ACTIVE);
+	const size_t smem = (size_t)bwd_stride(g->dim) * sizeof(double) + DX_ITEMS * 8 + 64;
+	if (!P.bytes || (g->nno + P.clen - 1) / P.clen > DX_ITEMS || smem > 200 * 1024) return SGI_OK;
+	cudaMemPool_t pool = nullptr;
+	int rc = scratch_pool(W, g->device, &pool);
+	if (rc) return rc;
+	void* buf = nullptr;
+	if (cudaMallocFromPoolAsync(&buf, P.bytes, pool, stream) != cudaSuccess) { cudaGetLastError(); return SGI_OK; }
+	PoolScratch hold;
+	hold.p = static_cast<char*>(buf);
+	hold.s = stream;
+	ListArgs la;
+	rc = launch_walk(W, P, &g, 0, 1, offs, x, nullptr, SGI_FP64, hold.p, stream, false, true, true, la);
+	if (rc) return rc;
+	void (*k)(ListArgs, const double*, double*) = R == 1 ? bwd_points_list_kernel<1> : R == 2 ? bwd_points_list_kernel<2>
+		: R == 4 ? bwd_points_list_kernel<4> : bwd_points_list_kernel<8>;
+	if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+	int blocks = 0;
+	rc = occupancy_grid(k, smem, W->sms, &blocks, 32 * DXW);
+	if (rc) return rc;
+	k<<<(int)std::min<long long>(blocks, npts), 32 * DXW, smem, stream>>>(la, gout, gx);
+	CUDA_TRY(cudaGetLastError());
+	g_stats.kernels += 2;
+	*done = true;
+	return SGI_OK;
+}
+
+} // namespace
+
 extern "C" int sgi_backward(sgi_grid_t g, long long npts, const double* x, const double* gout,
 	double* gx, double* gsurplus, void* stream_)
 {
@@ -3966,26 +4180,32 @@ extern "C" int sgi_backward(sgi_grid_t g, long long npts, const double* x, const
 	memset(&a, 0, sizeof(a));
 	a.G = desc_of(g, 0);
 	a.x = x; a.gout = gout; a.gx = gx; a.gs = gsurplus; a.npts = npts; a.dim = g->dim; a.TD = g->TD;
-	// a persistent launch over `items` warp-sized work items
-	auto launch = [&](void (*kern)(BwdArgs), size_t smem, long long items) -> int
+	// a persistent launch over `items` work items, `per` of them at a time per block
+	auto launch = [&](void (*kern)(BwdArgs), size_t smem, long long items, int threads = BLOCK, int per = WARPS) -> int
 	{
 		if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 		int blocks = 0;
-		int e = occupancy_grid(kern, smem, W->sms, &blocks);
+		int e = occupancy_grid(kern, smem, W->sms, &blocks, threads);
 		if (e) return e;
-		blocks = (int)std::min<long long>(blocks, (items + WARPS - 1) / WARPS);
+		blocks = (int)std::min<long long>(blocks, (items + per - 1) / per);
 		a.counter = W->counters + (W->next.fetch_add(1) % NCOUNTERS);
 		CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream));
-		kern<<<std::max(blocks, 1), BLOCK, smem, stream>>>(a);
+		kern<<<std::max(blocks, 1), threads, smem, stream>>>(a);
 		CUDA_TRY(cudaGetLastError());
 		g_stats.kernels++;
 		return SGI_OK;
 	};
 	if (!gsurplus)
 	{
-		void (*pk)(BwdArgs) = R == 1 ? bwd_points_kernel<1> : R == 2 ? bwd_points_kernel<2> : R == 4 ? bwd_points_kernel<4> : bwd_points_kernel<8>;
 		g_stats.points = npts;
-		return launch(pk, (size_t)WARPS * bwd_stride(g->dim) * sizeof(double), npts);
+		bool done = false;
+		rc = backward_lists(W, g, npts, x, gout, gx, R, stream, &done);
+		if (rc || done) return rc;
+		void (*pk)(BwdArgs) = R == 1 ? bwd_points_kernel<1> : R == 2 ? bwd_points_kernel<2> : R == 4 ? bwd_points_kernel<4> : bwd_points_kernel<8>;
+		// as many warps per block as their copies of the gradient leave room for
+		const size_t per_warp = (size_t)bwd_stride(g->dim) * sizeof(double);
+		const int warps = (int)std::max<size_t>(1, std::min<size_t>(WARPS, 200 * 1024 / per_warp));
+		return launch(pk, warps * per_warp, npts, warps * 32, warps);
 	}
 
 	// scratch (stream-ordered allocations from the device's pool)
@@ -4049,7 +4269,7 @@ extern "C" int sgi_backward(sgi_grid_t g, long long npts, const double* x, const
 	BWD_TRY(cudaMemsetAsync(gsurplus, 0, sizeof(double) * (size_t)g->nno * g->TD, stream));   // nodes without pairs
 	if (ntiles) BWD_RUN(launch(nk, 0, ntiles));
 	if (ntiles > 1) BWD_RUN(launch(bwd_join_kernel, 0, ntiles));
-	if (gx) BWD_RUN(launch(bwd_dx_kernel, (size_t)WARPS * 3 * g->dim * sizeof(double), npts));
+	if (gx) BWD_RUN(launch(bwd_dx_kernel, (size_t)(1 + 2 * DXW) * g->dim * sizeof(double), npts, 32 * DXW, 1));
 	cleanup();
 	g_stats.points = npts;
 	return SGI_OK;
@@ -4111,7 +4331,7 @@ extern "C" int sgi_interpolate_noalloc(int ngrids, const sgi_grid_t* grids, cons
 	}
 	const sgi_grid* g0 = grids[0];
 	const int variant = g_variant.load();   // resolved per group as sgi_interpolate does
-	if (fwd_smem(precision, g0->dim, true) > 200 * 1024) return fail(SGI_E_RANGE, "dim %d too large for shared staging", g0->dim);
+	if (dim_too_large(precision, g0->dim)) return fail(SGI_E_RANGE, "dim %d too large for shared staging", g0->dim);
 	// count the launches first: reject before launching anything
 	const int passes = (g0->TD + PASS - 1) / PASS;
 	long long launches = 0;

@@ -46,3 +46,25 @@ def test_backward_point_outside_every_support(cuda):
     assert torch.equal(gx, only) and bool(torch.isfinite(gx).all()) and bool(torch.isfinite(gs).all())
     keep = torch.arange(100, device="cuda") != 31
     assert torch.equal(gx[keep], ref[keep])
+
+
+@pytest.mark.parametrize("npts,nno", [(200, 3000), (145, 15_000)])
+def test_dx_alone_through_lists(cuda, npts, nno):
+    """dL/dx alone on a small batch is added from hit lists; here every node is
+    narrow in three of 48 dimensions, so that the lists' pool is sized for few
+    hits, and the points in the middle meet all nodes: the larger batch runs
+    out of room.  Either way the bits are those of both gradients' kernels."""
+    import itertools
+
+    import torch
+    rng = np.random.default_rng(4)
+    dims = np.array(list(itertools.islice(itertools.combinations(range(48), 3), nno - 1)))
+    idx = np.zeros((nno, 96), np.int32)
+    rows = np.arange(1, nno)[:, None]
+    idx[rows, dims], idx[rows, 48 + dims] = 64, 31
+    g = H.Grid(H.HostGrid.from_dense(idx, rng.standard_normal((nno, 40))))
+    X = np.full((npts, 48), 31 / 64) + rng.uniform(-0.5, 0.5, (npts, 48)) / 64
+    X[0], X[5, 7] = 0.9, np.nan
+    x = torch.from_numpy(X).cuda()
+    c = torch.from_numpy(rng.standard_normal((npts, 40))).cuda()
+    assert torch.equal(H.backward(g, x, c, want_surplus=False)[0], H.backward(g, x, c)[0])
