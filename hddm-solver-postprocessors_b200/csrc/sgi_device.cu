@@ -517,7 +517,7 @@ __device__ __forceinline__ void walk_lists(const GridDesc& G, const double* xs, 
 // FP64 form.  The walk only lists its hits (a window of 32 nodes holds two or
 // three of them); once 32 are listed, lane k takes hit k's weight, all lanes
 // busy, and the rows are then read QH at a time, QH such that a lane's loads
-// in flight fill 32 registers whatever the row width.  The adds follow the
+// in flight fill 32 registers (16 for rows of up to 64 outputs).  The adds follow the
 // list, which is in index order: gold's operations in gold's order.
 // Taking each window's hits at once instead (two rows in flight, the weights
 // of two or three busy lanes, then a wait for the rows) left the kernel
@@ -526,9 +526,12 @@ __device__ __forceinline__ void walk_lists(const GridDesc& G, const double* xs, 
 // outputs 5.4 against 3.2, 131,072 points on a 150,000-node grid of 256
 // outputs 17.9 against 15.3 ms, where the L2 now runs at 80 % of its peak.
 template <int V, int E>
-__global__ void __launch_bounds__(BLOCK, 4) fwd_f64_kernel(const __grid_constant__ FwdArgs a)
+__global__ void __launch_bounds__(BLOCK, V * E <= 2 ? 5 : 4) fwd_f64_kernel(const __grid_constant__ FwdArgs a)
 {
-	constexpr int QH = 16 / (V * E);
+	// narrow rows leave registers for a fifth block per SM, which hides more
+	// than twice the rows in flight per warp do (six ragged d=30 states of 64
+	// outputs 3.41 -> 3.25 ms, a regular grid of 32 outputs 9.20 -> 8.97 ms)
+	constexpr int QH = V * E <= 2 ? 8 / (V * E) : 16 / (V * E);
 	static_assert(32 % QH == 0, "groups of QH rows tile a full list");
 	extern __shared__ double smem[];
 	const int lane = threadIdx.x & 31;
