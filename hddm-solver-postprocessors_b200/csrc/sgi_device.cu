@@ -7,7 +7,8 @@
 // subtree is the index range [n, skip[n]).
 //
 // Forward kernels: one warp per query point, points pulled from a device work
-// counter.  Two walks find a point's active nodes.
+// counter; small batches spread a point over many warps (walk_chunks_kernel).
+// Two walks find a point's active nodes.
 //
 // Window walk (FP64 form, hit counts, backward, FP32C fallback): the warp
 // walks the nodes in windows of 32 consecutive indices:
@@ -15,8 +16,8 @@
 //     component in which it differs from its parent);
 //   * an inclusive max-scan of the skip pointers of failing nodes marks every
 //     node inside a failing node's subtree as pruned;
-//   * surviving nodes ("hits") get their weight, the product of all their
-//     hats in dimension order, from their own lane;
+//   * surviving nodes ("hits") are listed; 32 at a time, they get their
+//     weights, the product of all their hats in dimension order, a lane each;
 //   * hits are accumulated in index order: all lanes read the node's surplus
 //     row (coalesced) and update the TotalDof accumulators they own;
 //   * the next window starts after the window or after the largest pruned
@@ -458,7 +459,12 @@ __device__ __forceinline__ void load_row(const float* row, int o, bool in, float
 template <int E>
 __device__ __forceinline__ void load_ahead(const double* row, double* d)
 {
-	if (E == 2) asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(d[0]), "=d"(d[E - 1]) : "l"(row));
+	if constexpr (E >= 2)
+	{
+#pragma unroll
+		for (int e = 0; e < E; e += 2)
+			asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(d[e]), "=d"(d[e + 1]) : "l"(row + e));
+	}
 	else asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(d[0]) : "l"(row));
 }
 
@@ -915,13 +921,15 @@ __device__ __forceinline__ uint4 pack_seg(uint32_t b, uint32_t e, double w)
 
 // QV: fine rows per group at eight outputs per lane; narrower rows take more,
 // up to FLUSH, so that a lane's loads in flight fill as many registers.
+// MINB: blocks per SM to compile for; the variant of two has room for a third
+// on rows of up to 64 outputs.
 template <int V, int E, int QV, int MINB, bool FULLROW>
-__global__ void __launch_bounds__(BLOCK, MINB) fwd_f32d_kernel(const __grid_constant__ FwdArgs a)
+__global__ void __launch_bounds__(BLOCK, MINB == 2 && V * E <= 2 ? 3 : MINB) fwd_f32d_kernel(const __grid_constant__ FwdArgs a)
 {
 	constexpr int Q = QV * 8 / (V * E) < FLUSH ? QV * 8 / (V * E) : FLUSH;
 	// big rows per group: 32 registers of loads in flight, 64 in the variant
-	// of fewer warps
-	constexpr int QB0 = (MINB == 2 ? 32 : 16) / (V * E);
+	// of fewer warps (16 where that variant's third block fits beside them)
+	constexpr int QB0 = (MINB == 2 ? (V * E == 2 ? 8 : 32) : 16) / (V * E);
 	constexpr int QB = QB0 < 8 ? QB0 : 8;
 	constexpr bool LISTB = V * E <= LISTB_MAX;
 	static_assert(QB >= 2 && 31 + QB <= BCAP, "the big-term list holds a remainder and a step's hits");
@@ -1113,29 +1121,51 @@ __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32d_kernel(const __grid_cons
 					if (since >= FLUSH) { flush(); since = 0; }
 				}
 			};
-			// big-term list entries [h, hend), N at a time
-			auto bigs = [&](auto n, int h, int hend)
+			// columns past the row's end read this lane's first (not stored)
+			auto big_row = [&](uint32_t row, double (*d)[E])
 			{
-				constexpr int N = decltype(n)::value;
-				for (; h + N <= hend; h += N)
-				{
-					double sv[N][V][E], wq[N];
+				const double* r = s64l + (size_t)row * ld;
 #pragma unroll
-					for (int q = 0; q < N; q++)
+				for (int v = 0; v < V; v++) load_ahead<E>(r + (FULLROW || lcol + v * 32 * E < (int)ld ? v * 32 * E : 0), d[v]);
+			};
+			// big-term list entries [0, n), QB at a time; the last group may be
+			// short (its rows past n are its last again, and are not added)
+			auto bigs = [&](int n)
+			{
+				int h = 0;
+				for (; h + QB <= n; h += QB)
+				{
+					double sv[QB][V][E], wq[QB];
+#pragma unroll
+					for (int q = 0; q < QB; q++)
 					{
 						const uint4 t = fb[h + q];
 						wq[q] = __hiloint2double((int)t.w, (int)t.z);
-						const double* row = s64l + (size_t)t.x * ld;
-#pragma unroll
-						for (int v = 0; v < V; v++)
-							load_row<E>(row, v * 32 * E, FULLROW || lcol + v * 32 * E < (int)ld, sv[q][v]);
+						big_row(t.x, sv[q]);
 					}
 #pragma unroll
-					for (int q = 0; q < N; q++)
+					for (int q = 0; q < QB; q++)
 #pragma unroll
 						for (int v = 0; v < V; v++)
 #pragma unroll
 							for (int e = 0; e < E; e++) acc[v][e] = fma(wq[q], sv[q][v][e], acc[v][e]);
+				}
+				if (h < n)
+				{
+					double sv[QB][V][E];
+#pragma unroll
+					for (int q = 0; q < QB; q++) big_row(fb[min(h + q, n - 1)].x, sv[q]);
+#pragma unroll
+					for (int q = 0; q < QB; q++)
+					{
+						if (h + q >= n) break;   // warp-uniform
+						const uint4 t = fb[h + q];
+						const double wq = __hiloint2double((int)t.w, (int)t.z);
+#pragma unroll
+						for (int v = 0; v < V; v++)
+#pragma unroll
+							for (int e = 0; e < E; e++) acc[v][e] = fma(wq, sv[q][v][e], acc[v][e]);
+					}
 				}
 			};
 			while (size > 0)
@@ -1233,7 +1263,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32d_kernel(const __grid_cons
 						{
 							// all whole groups; the remainder (< QB entries) moves to the front
 							__syncwarp();
-							bigs(std::integral_constant<int, QB>(), 0, wholeb);
+							bigs(wholeb);
 							const int rem = cntb - wholeb;
 							uint4 t = make_uint4(0u, 0u, 0u, 0u);
 							if (lane < rem) t = fb[wholeb + lane];
@@ -1306,7 +1336,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32d_kernel(const __grid_cons
 			if (cntb)
 			{
 				__syncwarp();
-				bigs(std::integral_constant<int, 1>(), 0, cntb);
+				bigs(cntb);
 			}
 			if (cnt)
 			{
@@ -2749,16 +2779,20 @@ int lane_outputs(int ld, int cols) { return ld <= 32 ? 1 : cols <= 64 ? 2 : cols
 // as a narrow row's adds hide less (d=59 and d=30 grids of 60,000 to 150,000
 // nodes; us for variants 0 / 1 / 2.  256 outputs: 10,007 points 624 / 747 /
 // 576, 20,000 990 / 1,104 / 986, 40,000 1,792 / 1,772 / 1,821.  118 outputs:
-// 5,000 491 / 609 / 444, 10,007 573 / 641 / 603, 20,000 912 / 968 / 976,
-// 40,000 1,627 / 1,568 / 1,780.  64 outputs: 2,000 155 / 157 / 146, 5,000
-// 174 / 173 / 194).
-int auto_variant(int variant, long long npts, int sms, int outputs)
+// 4,000 264 / 327 / 246, 7,500 306 / 371 / 341, 20,000 912 / 968 / 976, 40,000
+// 1,627 / 1,568 / 1,780.  64 outputs: 4,000 230 / 235 / 214, 7,500 274 / 264 /
+// 245, 15,000 418 / 362 / 366.  32 outputs: 4,000 198 / 206 / 196, 7,500 230 /
+// 233 / 226, 15,000 339 / 314 / 336).
+// Wide rows: the line falls with the hits per point, too (15,000 points of 200
+// outputs: a 60,000-node d=45 grid of 440 active nodes 682 for 1 and 613 for
+// 2, a 40,000-node d=16 grid of 250 215 and 238).
+int auto_variant(int variant, long long npts, int sms, int outputs, double mean_active)
 {
 	if (variant >= 0) return variant;
 	const long long per_sm = npts / sms;
-	if (outputs == 8) return per_sm < 128 ? 2 : 1;
-	if (outputs == 4) return per_sm < 48 ? 2 : per_sm < 256 ? 0 : 1;
-	return per_sm < 16 ? 2 : 1;
+	if (outputs == 8) return (double)per_sm < std::min(128.0, std::max(80.0, mean_active / 4)) ? 2 : 1;
+	if (outputs == 4) return per_sm < 36 ? 2 : per_sm < 256 ? 0 : 1;
+	return per_sm < (outputs == 2 ? 64 : 32) ? 2 : 1;
 }
 
 uint32_t float_bits(float f)
@@ -3034,8 +3068,10 @@ int build_image(const HostGrid& g, unsigned flags, GridImage& im)
 	im.rec = L.rec; im.comps = L.comps; im.coarse_index = L.lo_index; im.parent = L.parent; im.aux = L.aux;
 	im.parent_h = L.parent;
 	// a node's share of the unit cube is the product of its supports' lengths,
-	// (min(i, j + 1) - max(0, j - 1)) / i
-	for (int n = 0; n < g.nno; n++)
+	// (min(i, j + 1) - max(0, j - 1)) / i; the sum over at most 8,192 evenly
+	// spaced nodes serves, as it only sizes scratch and picks kernels
+	const int step = std::max(1, g.nno / 8192);
+	for (int n = 0; n < g.nno; n += step)
 	{
 		const uint32_t* r = &L.rec[4 * (size_t)n];
 		if (r[2] & NODE_DEAD) continue;
@@ -3048,7 +3084,7 @@ int build_image(const HostGrid& g, unsigned flags, GridImage& im)
 			num *= std::max(0, std::min(i, j + 1) - std::max(0, j - 1));
 			den *= i;
 		}
-		if (den < 1e300) im.mean_active += num / den;
+		if (den < 1e300) im.mean_active += step * (num / den);
 	}
 	im.skip_h.resize(g.nno);
 	im.depth_h.resize(g.nno);
@@ -3613,6 +3649,14 @@ int group_clen(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng, con
 	                 : (chunk >= maxnno ? 0 : chunk);
 }
 
+// Active nodes per point of a launch group, expected for uniform points.
+double mean_active(const sgi_grid_t* grids, int gb, int ng, const long long* pt_offsets)
+{
+	double a = 0.0;
+	for (int k = 0; k < ng; k++) a += (double)(pt_offsets[gb + k + 1] - pt_offsets[gb + k]) * grids[gb + k]->mean_active;
+	return a / (double)std::max(1ll, pt_offsets[gb + ng] - pt_offsets[gb]);
+}
+
 // How a launch group's points run in two phases.
 struct ListPlan
 {
@@ -3872,6 +3916,7 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 		const int clen = group_clen(W, grids, gb, ng, pt_offsets, precision, chunk);
 		const int nchunks = clen ? (maxnno + clen - 1) / clen : 1;
 		const bool descent = precision == SGI_FP32C && descent_ok(grids, gb, ng, clen > 0);
+		const double active = mean_active(grids, gb, ng, pt_offsets);
 		const bool small = a.npts < (long long)W->sms * WARPS;
 		// small unchunked FP64 batches: one warp per (point, 32 outputs)
 		const bool cols_mode = precision == SGI_FP64 && small && clen == 0;
@@ -3889,7 +3934,7 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 			const size_t smem = cols_mode ? (size_t)WARPS * cols_stride(g0->dim) * sizeof(double)
 			                              : fwd_smem(precision, g0->dim, descent, outputs);
 			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel
-				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, W->sms, outputs), descent);
+				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, W->sms, outputs, active), descent);
 			if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 			int blocks = 0;
 			rc = occupancy_grid(kern, smem, W->sms, &blocks);
@@ -4367,6 +4412,7 @@ extern "C" int sgi_interpolate_noalloc(int ngrids, const sgi_grid_t* grids, cons
 		set_starts(a, grids, gb, ng);   // whole grids: the roots' groups
 		// the kernels sgi_interpolate picks for an unchunked launch
 		const bool descent = precision == SGI_FP32C && descent_ok(grids, gb, ng, false);
+		const double active = mean_active(grids, gb, ng, pt_offsets);
 		const bool small = a.npts < (long long)sms * WARPS;
 		const bool cols_mode = precision == SGI_FP64 && small;
 		for (int ob = 0; ob < g0->TD; ob += PASS)
@@ -4379,7 +4425,7 @@ extern "C" int sgi_interpolate_noalloc(int ngrids, const sgi_grid_t* grids, cons
 			const size_t smem = cols_mode ? (size_t)WARPS * cols_stride(g0->dim) * sizeof(double)
 			                              : fwd_smem(precision, g0->dim, descent, outputs);
 			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel
-				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, sms, outputs), descent);
+				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, sms, outputs, active), descent);
 			if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 			int blocks = 0;
 			rc = occupancy_grid(kern, smem, sms, &blocks);

@@ -325,9 +325,10 @@ int sgi_set_chunk_rows(int rows);
  * so their results may differ in the last bits (all within the FP32C
  * tolerance).  variant < 0 or SGI_FP32C_AUTO restores the default,
  * automatic by the points per SM and the width of a launch's rows: above 128
- * outputs 2 for fewer than 128 points per SM (18,944 on a B200), else 1; above
- * 64 outputs 2 for fewer than 48, 0 for fewer than 256, else 1; below, 2 for
- * fewer than 16, else 1.  Returns the previous setting
+ * outputs 2 for fewer points per SM than a quarter of the grids' mean active
+ * nodes (at least 80, at most 128), else 1; above 64 outputs 2 for fewer than
+ * 36, 0 for fewer than 256, else 1; above 32 outputs 2 for fewer than 64, else
+ * 1; below, 2 for fewer than 32, else 1.  Returns the previous setting
  * (SGI_FP32C_AUTO for automatic), or a negative error code.  No reference
  * counterpart. */
 #define SGI_FP32C_AUTO 255

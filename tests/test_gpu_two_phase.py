@@ -76,3 +76,21 @@ def test_pool_that_runs_out(cuda, npts, nno, td):
     X[0] = 0.9
     g = H.Grid(H.HostGrid.from_dense(idx, sur))
     assert np.array_equal(_run(g, X), O.Gold(idx, sur).interpolate(X, nthreads=4))
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2])
+@pytest.mark.parametrize("td", [20, 33, 64, 65, 118, 128])
+def test_fp32c_big_term_lists(cuda, td, variant):
+    """Narrow rows list their big terms: points of no, a few and hundreds of
+    big terms (surpluses that do not decay with the level make every term
+    big), whole and short groups, against the oracle."""
+    idx, sur = H.HostGrid.adaptive(14, 3000, td, seed=td).arrays()
+    X = H.gen_points(14, 1500, kind=2, seed=3)
+    prev = H.set_fp32c_variant(variant)
+    try:
+        for s in (sur, np.sign(sur) * (0.5 + np.abs(sur) / (1 + np.abs(sur).max()))):
+            g = H.Grid(H.HostGrid.from_dense(idx, s), flags=H.BUILD_FP32)
+            err = O.rel_error(_run(g, X, H.FP32C), O.Gold(idx, s).interpolate(X, nthreads=4))[0]
+            assert err <= FP32C_TOL
+    finally:
+        H.set_fp32c_variant(prev)
