@@ -2245,12 +2245,13 @@ __device__ __forceinline__ void dx_pass(const GridDesc& G, const double* xs, dou
 					const uint2 cc = q < 16u ? c[u] : __ldg(G.comps + cp + q);
 					const double xd = xs[cc.x];
 					const double i = u32_to_double(cc.y & 0xffffu), j = u32_to_double(cc.y >> 16);
-					// slope -i sign(x i - j): i's sign bit from the difference
+					// slope -i sign(x i - j): i's sign bit from the difference; 0 at
+					// the hat's centre (and added there, as cs may not be finite)
 					const double t = fma(xd, i, -j);
-					const double slope = __hiloint2double(__double2hiint(i) | (~__double2hiint(t) & 0x80000000), __double2loint(i));
+					const double side = __hiloint2double(__double2hiint(i) | (~__double2hiint(t) & 0x80000000), __double2loint(i));
+					const double slope = t != 0.0 ? side : 0.0;
 					const double h = __dsub_rn(1.0, fabs(__dsub_rn(__dmul_rn(xd, i), j)));   // as hat()
-					const double v = a * slope * rcp_hat(h);
-					if (t != 0.0) gh[cc.x] += v;
+					gh[cc.x] += a * slope * rcp_hat(h);
 				}
 				__syncwarp();
 				q += 16;

@@ -48,6 +48,25 @@ def test_backward_point_outside_every_support(cuda):
     assert torch.equal(gx[keep], ref[keep])
 
 
+def test_nan_gout_at_hat_centres(cuda):
+    """A NaN in dL/dvalue reaches dL/dx also where the slope is 0: at the
+    origin every active non-constant hat is at its centre.  NaN in the same
+    places as in the oracle, in both entry forms."""
+    import torch
+    hg = H.HostGrid.adaptive(10, 500, 40, seed=3)
+    X = H.gen_points(10, 100, kind=0, seed=4, kink_reject=1e-6)
+    X[7] = 0.0
+    C = np.random.default_rng(5).standard_normal((100, 40))
+    C[[7, 8], [3, 39]] = np.nan
+    ox = O.Gold(*hg.arrays()).gradient(X, C)[0]
+    assert np.isnan(ox[7]).any()
+    g = H.Grid(hg)
+    x, c = torch.from_numpy(X).cuda(), torch.from_numpy(C).cuda()
+    for want in (True, False):
+        gx = H.backward(g, x, c, want_surplus=want)[0].cpu().numpy()
+        assert np.array_equal(np.isnan(gx), np.isnan(ox))
+
+
 @pytest.mark.parametrize("npts,nno", [(200, 3000), (145, 15_000)])
 def test_dx_alone_through_lists(cuda, npts, nno):
     """dL/dx alone on a small batch is added from hit lists; here every node is
