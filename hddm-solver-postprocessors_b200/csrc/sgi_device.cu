@@ -2080,10 +2080,11 @@ struct BwdArgs
 	uint32_t* pair_idx;
 	const uint32_t* sorted_node; // sorted by node: node, pair number
 	const uint32_t* sorted_idx;
-	double* part;                // sums of nodes cut by tile ends, 2 per tile of PART pairs
+	double* part;                // sums of nodes cut by tile ends, 2 per tile
 	unsigned long long* counter;
 	long long npts, npairs;
 	int dim, TD;
+	int tile;                    // pairs per tile
 };
 
 // Sums of C values per lane over the warp: lane l gets value l >> (5 - log2 C).
@@ -2464,47 +2465,59 @@ __global__ void __launch_bounds__(BLOCK) bwd_list_kernel(const __grid_constant__
 	}
 }
 
-// dL/dsurplus and the pairs' cs * w: the sorted pairs are cut into tiles of
-// PART, one warp each, so that a node of many pairs (the root is active for
-// every point) is spread over warps and one of few costs no start-up: the rows
-// stream through, QB at a time, across node boundaries.  A node's sum goes to
-// gs when the tile holds all its pairs, else to `part`: the tile's first node
-// when it began before the tile to sum 2 t, a node that goes on after it to
-// sum 2 t + 1 (2 t when it covers the tile's first pair); bwd_join_kernel adds
-// them in order.  Pair numbers are loaded two batches of 32 ahead, the pairs
-// they name one ahead.
-constexpr long long PART = 1024;
+// dL/dsurplus and the pairs' cs * w: the sorted pairs are cut into tiles, one
+// warp each, so that a node of many pairs (the root is active for every point)
+// is spread over warps and one of few costs no start-up: the rows stream
+// through, QB at a time, across node boundaries.  A node's sum goes to gs when
+// the tile holds all its pairs, else to `part`: the tile's first node when it
+// began before the tile to sum 2 t, a node that goes on after it to sum 2 t + 1
+// (2 t when it covers the tile's first pair); bwd_join_kernel adds them in
+// order.  Pair numbers are loaded two batches of 32 ahead, the pairs they name
+// one ahead.  Where nodes begin among a group's rows (most groups of a small
+// batch), the gout rows and the beginning nodes' surplus rows of QS pairs are
+// loaded together, then the sums are split.
+//
+// A tile's length follows from the number of pairs alone (so do the bits):
+// about TILES tiles, a little more than the warps that the GPU holds (half or
+// four times as many: within 3 % on average over 399 calls), of at most
+// TILE_MAX pairs, where a tile's start-up and its parts no longer show.  With
+// TILE_MAX pairs at every size, and one row at a time where nodes begin, both
+// gradients of 200 points of a 20,000-node d=10 grid of 118 outputs took 533
+// us, now 186, and 1,000 points of a 100,000-node d=59 grid 1,180, now 720;
+// 32,768 points of 300,000 nodes, 128 outputs, take 5.8 ms either way.
+constexpr long long TILES = 4096;
+constexpr long long TILE_MAX = 1024;
+
+long long tile_pairs(long long npairs)
+{
+	return std::min(TILE_MAX, std::max(32ll, (npairs / TILES + 31) / 32 * 32));
+}
 
 template <int R, bool DOT, bool VEC>
 __global__ void __launch_bounds__(BLOCK, R == 8 ? 2 : 3) bwd_nodes_kernel(const __grid_constant__ BwdArgs a)
 {
-	constexpr int QB = RowGroup<R>::QB, CB = RowGroup<R>::CB;
+	// rows read 8 bytes at a time need registers for their column tests
+	constexpr int CB = RowGroup<R>::CB, QB = VEC || R == 1 || R == 8 ? RowGroup<R>::QB : RowGroup<R>::QB / 2;
+	constexpr int QS = R >= 4 ? 1 : R == 2 ? 2 : 4;
 	__shared__ PairVal batch[WARPS][32];   // this batch's pairs: one 16-byte read per row instead of three shuffles
 	const int lane = threadIdx.x & 31;
 	PairVal* pairs = batch[threadIdx.x >> 5];
 	const GridDesc& G = a.G;
 	const int TD = a.TD;
 	const uint32_t ld = (uint32_t)a.TD;
-	const long long ntiles = (a.npairs + PART - 1) / PART;
+	const long long ntiles = (a.npairs + a.tile - 1) / a.tile;
 	for (;;)
 	{
 		long long it = 0;
 		if (lane == 0) it = (long long)atomicAdd(a.counter, 1ull);
 		it = __shfl_sync(FULL, it, 0);
 		if (it >= ntiles) break;
-		const long long tb = it * PART, te = min(tb + PART, a.npairs);
+		const long long tb = it * a.tile, te = min(tb + a.tile, a.npairs);
 		uint32_t cur = __ldg(a.sorted_node + tb);
 		bool carried = tb > 0 && __ldg(a.sorted_node + tb - 1) == cur;   // began before the tile
 		const bool goes_on = te < a.npairs && __ldg(a.sorted_node + te) == __ldg(a.sorted_node + te - 1);
 		bool at_start = true;                                            // `cur` covers the tile's first pair
 		double mul[R], acc[R];
-		auto begin = [&](uint32_t n)
-		{
-			cur = n;
-			if (DOT) bwd_row<R, true>(G.s64 + (size_t)n * G.ld, G.ld, lane, mul);
-#pragma unroll
-			for (int r = 0; r < R; r++) acc[r] = 0.0;
-		};
 		auto store = [&](double* dst)
 		{
 #pragma unroll
@@ -2514,7 +2527,9 @@ __global__ void __launch_bounds__(BLOCK, R == 8 ? 2 : 3) bwd_nodes_kernel(const 
 				if (o < TD) dst[o] = acc[r];
 			}
 		};
-		begin(cur);
+		if (DOT) bwd_row<R, true>(G.s64 + (size_t)cur * G.ld, G.ld, lane, mul);
+#pragma unroll
+		for (int r = 0; r < R; r++) acc[r] = 0.0;
 		uint32_t node1 = 0u, idx1 = 0u, node2 = 0u, idx2 = 0u;   // this batch's, the next one's
 		PairVal pv1{ 0.0, 0u, 0u };
 		if (tb + lane < te)
@@ -2581,28 +2596,55 @@ __global__ void __launch_bounds__(BLOCK, R == 8 ? 2 : 3) bwd_nodes_kernel(const 
 					}
 					continue;
 				}
-				// a node begins among these rows, or fewer than CB are left: one at a time
-				for (int q = k; q < min(k + CB, m); q++)
+				// nodes begin among these rows, or fewer than CB are left
+#pragma unroll 1
+				for (int h = k; h < min(k + CB, m); h += QS)
 				{
-					if ((bounds >> q) & 1u)
-					{
-						store(at_start && carried ? a.part + (size_t)(2 * it) * TD : a.gs + (size_t)cur * TD);
-						at_start = false;
-						begin(__shfl_sync(FULL, node, q));
-					}
-					const double wq = pairs[q].w;
-					double v[R], c[1] = { 0.0 };
-					bwd_row<R, VEC>(a.gout + (size_t)pairs[q].point * ld, TD, lane, v);
+					double v[QS][R], sv[QS][R], c[QS], wq[QS];
+					// one row at a time: the node's row goes where it is needed
+					constexpr bool ONE = QS == 1;
 #pragma unroll
-					for (int r = 0; r < R; r++)
+					for (int q = 0; q < QS; q++)
 					{
-						acc[r] = fma(wq, v[r], acc[r]);
-						if (DOT) c[0] = fma(mul[r], v[r], c[0]);
+						const int i = min(h + q, m - 1);
+						const PairVal pq = pairs[i];
+						wq[q] = pq.w;
+						bwd_row<R, VEC>(a.gout + (size_t)pq.point * ld, h + q < m ? TD : 0, lane, v[q]);
+						if (DOT && !ONE)
+						{
+							const uint32_t n = __shfl_sync(FULL, node, i);
+							if ((bounds >> i) & 1u) bwd_row<R, true>(G.s64 + (size_t)n * G.ld, G.ld, lane, sv[q]);
+						}
+					}
+#pragma unroll
+					for (int q = 0; q < QS; q++)
+					{
+						c[q] = 0.0;
+						if (h + q >= m) continue;   // warp-uniform
+						if ((bounds >> (h + q)) & 1u)
+						{
+							store(at_start && carried ? a.part + (size_t)(2 * it) * TD : a.gs + (size_t)cur * TD);
+							at_start = false;
+							cur = __shfl_sync(FULL, node, h + q);
+							if (DOT && ONE) bwd_row<R, true>(G.s64 + (size_t)cur * G.ld, G.ld, lane, mul);
+#pragma unroll
+							for (int r = 0; r < R; r++)
+							{
+								acc[r] = 0.0;
+								if (DOT && !ONE) mul[r] = sv[q][r];
+							}
+						}
+#pragma unroll
+						for (int r = 0; r < R; r++)
+						{
+							acc[r] = fma(wq[q], v[q][r], acc[r]);
+							if (DOT) c[q] = fma(mul[r], v[q][r], c[q]);
+						}
 					}
 					if (DOT)
 					{
-						const double t = warp_sums<1>(c, lane);   // every lane has the sum
-						if (lane == q) dot = t;
+						const double u = __shfl_sync(FULL, warp_sums<QS>(c, lane), (lane & (QS - 1)) * (32 / QS));
+						if (lane - h >= 0 && lane - h < QS) dot = u;
 					}
 				}
 			}
@@ -2613,17 +2655,19 @@ __global__ void __launch_bounds__(BLOCK, R == 8 ? 2 : 3) bwd_nodes_kernel(const 
 	}
 }
 
-// Nodes cut by tile ends: their parts' sums, added in order, by the warp of
-// the tile in which the node begins.
+// Nodes cut by tile ends: their parts' sums, added in order, by a warp per
+// (tile in which the node begins, 32 outputs).
 __global__ void __launch_bounds__(BLOCK) bwd_join_kernel(const __grid_constant__ BwdArgs a)
 {
 	const int lane = threadIdx.x & 31;
 	const uint32_t* key = a.sorted_node;
-	const long long ntiles = (a.npairs + PART - 1) / PART;
-	for (long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t + 1 < ntiles;
-	     t += ((long long)gridDim.x * blockDim.x) >> 5)   // warp-uniform
+	const long long ntiles = (a.npairs + a.tile - 1) / a.tile;
+	const int ncb = (a.TD + 31) / 32;
+	for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < (ntiles - 1) * ncb;
+	     i += ((long long)gridDim.x * blockDim.x) >> 5)   // warp-uniform
 	{
-		const long long tb = t * PART, te = tb + PART;
+		const long long t = i / ncb;
+		const long long tb = t * a.tile, te = tb + a.tile;
 		const uint32_t n = __ldg(key + te - 1);
 		const bool covers = __ldg(key + tb) == n;
 		if (__ldg(key + te) != n || (covers && tb > 0 && __ldg(key + tb - 1) == n)) continue;
@@ -2631,14 +2675,24 @@ __global__ void __launch_bounds__(BLOCK) bwd_join_kernel(const __grid_constant__
 		for (unsigned on = FULL; on == FULL;)
 		{
 			const long long u = last + 1 + lane;
-			on = __ballot_sync(FULL, u < ntiles && __ldg(key + u * PART) == n);   // a run of low lanes
+			on = __ballot_sync(FULL, u < ntiles && __ldg(key + u * a.tile) == n);   // a run of low lanes
 			last += __popc(on);
 		}
-		for (int o = lane; o < a.TD; o += 32)
+		const int o = (int)(i % ncb) * 32 + lane;
+		if (o < a.TD)
 		{
 			double s = a.part[(size_t)(2 * t + (covers ? 0 : 1)) * a.TD + o];
-#pragma unroll 4
-			for (long long u = t + 1; u <= last; u++) s += a.part[(size_t)(2 * u) * a.TD + o];
+			const double* part = a.part + (size_t)(2 * (t + 1)) * a.TD + o;
+			long long m = last - t;   // parts left
+			for (; m >= 16; m -= 16, part += (size_t)32 * a.TD)
+			{
+				double v[16];
+#pragma unroll
+				for (int j = 0; j < 16; j++) asm volatile("ld.global.f64 %0, [%1];" : "=d"(v[j]) : "l"(part + (size_t)(2 * j) * a.TD));
+#pragma unroll
+				for (int j = 0; j < 16; j++) s += v[j];
+			}
+			for (; m > 0; m--, part += (size_t)2 * a.TD) s += *part;
 			a.gs[(size_t)n * a.TD + o] = s;
 		}
 	}
@@ -4230,6 +4284,7 @@ extern "C" int sgi_backward(sgi_grid_t g, long long npts, const double* x, const
 	a.G = desc_of(g, 0);
 	a.x = x; a.gout = gout; a.gx = gx; a.gs = gsurplus; a.npts = npts; a.dim = g->dim; a.TD = g->TD;
 	// a persistent launch over `items` work items, `per` of them at a time per block
+	int blocks_of_last = 0;
 	auto launch = [&](void (*kern)(BwdArgs), size_t smem, long long items, int threads = BLOCK, int per = WARPS) -> int
 	{
 		if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -4239,8 +4294,10 @@ extern "C" int sgi_backward(sgi_grid_t g, long long npts, const double* x, const
 		blocks = (int)std::min<long long>(blocks, (items + per - 1) / per);
 		a.counter = W->counters + (W->next.fetch_add(1) % NCOUNTERS);
 		CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream));
-		kern<<<std::max(blocks, 1), threads, smem, stream>>>(a);
+		blocks = std::max(blocks, 1);
+		kern<<<blocks, threads, smem, stream>>>(a);
 		CUDA_TRY(cudaGetLastError());
+		blocks_of_last = blocks;
 		g_stats.kernels++;
 		return SGI_OK;
 	};
@@ -4292,7 +4349,8 @@ extern "C" int sgi_backward(sgi_grid_t g, long long npts, const double* x, const
 	a.npairs = npairs;
 	a.pair_off = offs;
 	uint32_t *node_sorted = nullptr, *idx_sorted = nullptr;
-	const long long ntiles = (npairs + PART - 1) / PART;
+	a.tile = (int)tile_pairs(npairs);
+	const long long ntiles = (npairs + a.tile - 1) / a.tile;
 	BWD_TRY(take(&a.pair_node, 4 * (size_t)npairs));
 	BWD_TRY(take(&a.pair_val, sizeof(PairVal) * (size_t)npairs));
 	BWD_TRY(take(&a.pair_idx, 4 * (size_t)npairs));
@@ -4316,8 +4374,15 @@ extern "C" int sgi_backward(sgi_grid_t g, long long npts, const double* x, const
 	void (*nk)(BwdArgs) = R == 1 ? nodes_kernel<1>(gx, vec) : R == 2 ? nodes_kernel<2>(gx, vec)
 		: R == 4 ? nodes_kernel<4>(gx, vec) : nodes_kernel<8>(gx, vec);
 	BWD_TRY(cudaMemsetAsync(gsurplus, 0, sizeof(double) * (size_t)g->nno * g->TD, stream));   // nodes without pairs
-	if (ntiles) BWD_RUN(launch(nk, 0, ntiles));
-	if (ntiles > 1) BWD_RUN(launch(bwd_join_kernel, 0, ntiles));
+	if (ntiles)
+	{
+		// few tiles: blocks of two warps, which spread over more SMs
+		const int warps = ntiles < (long long)W->sms * WARPS * 2 ? 2 : WARPS;
+		BWD_RUN(launch(nk, 0, ntiles, warps * 32, warps));
+		g_stats.grid_blocks = blocks_of_last;
+		g_stats.block_threads = warps * 32;
+	}
+	if (ntiles > 1) BWD_RUN(launch(bwd_join_kernel, 0, (ntiles - 1) * ((g->TD + 31) / 32)));
 	if (gx) BWD_RUN(launch(bwd_dx_kernel, (size_t)(1 + 2 * DXW) * g->dim * sizeof(double), npts, 32 * DXW, 1));
 	cleanup();
 	g_stats.points = npts;
