@@ -1393,29 +1393,33 @@ __device__ __forceinline__ bool keeps_term(const GridDesc& G, uint32_t flags, fl
 	return ((flags & NODE_COARSE) && bound >= G.big_below) || bound >= G.skip_below;
 }
 
-// Output `col` of a point, walked and added by this warp alone (lane l's
-// column is l's own): phase 2's way with a point whose lists found no room.
-// lw, ln: CLIST entries of shared memory.
-template <int DEPTH>
-__device__ __forceinline__ double walk_column(const GridDesc& G, const double* xs, double* lw, uint32_t* ln, int lane,
-	int col, bool cin)
+// Outputs col .. col + E - 1 of a point, walked and added by this warp alone
+// (each lane has its own), one walk for all of them: the way of
+// fwd_f64_cols_kernel, and phase 2's way with a point whose lists found no
+// room.  lw, ln: CLIST entries of shared memory.
+template <int E, int DEPTH>
+__device__ __forceinline__ void walk_columns(const GridDesc& G, const double* xs, double* lw, uint32_t* ln, int lane,
+	int col, bool cin, double* acc)
 {
-	double acc = 0.0;
+#pragma unroll
+	for (int e = 0; e < E; e++) acc[e] = 0.0;
 	int n = 0;
 	// list entries [0, cnt) in order
 	auto drain = [&](int cnt)
 	{
 		for (int b = 0; b < cnt; b += DEPTH)
 		{
-			double sv[DEPTH];
+			double sv[DEPTH][E];
 #pragma unroll
 			for (int q = 0; q < DEPTH; q++)
-				sv[q] = (b + q < cnt && cin) ? __ldg(G.s64 + (size_t)ln[b + q] * G.ld + col) : 0.0;
+				load_row<E>(G.s64 + (b + q < cnt && cin ? (size_t)ln[b + q] * G.ld : 0), col, b + q < cnt && cin, sv[q]);
 #pragma unroll
 			for (int q = 0; q < DEPTH; q++)
 			{
 				if (b + q >= cnt) break;   // warp-uniform
-				acc = __dadd_rn(acc, __dmul_rn(lw[b + q], sv[q]));
+				const double wq = lw[b + q];
+#pragma unroll
+				for (int e = 0; e < E; e++) acc[e] = __dadd_rn(acc[e], __dmul_rn(wq, sv[q][e]));
 			}
 		}
 	};
@@ -1440,7 +1444,6 @@ __device__ __forceinline__ double walk_column(const GridDesc& G, const double* x
 		}
 	});
 	if (n) drain(n);
-	return acc;
 }
 
 __global__ void __launch_bounds__(BLOCK) fwd_f64_cols_kernel(const __grid_constant__ FwdArgs a)
@@ -1465,7 +1468,8 @@ __global__ void __launch_bounds__(BLOCK) fwd_f64_cols_kernel(const __grid_consta
 		const bool cin = col < cols;
 		const GridDesc& G = a.g[find_grid(a, p)];
 		const bool ok = load_point(a, p, xs, lane);
-		const double acc = ok ? walk_column<CDEPTH>(G, xs, lw, ln, lane, a.o_begin + col, cin) : 0.0;
+		double acc = 0.0;
+		if (ok) walk_columns<1, CDEPTH>(G, xs, lw, ln, lane, a.o_begin + col, cin, &acc);
 		if (cin)
 			a.out[(size_t)p * a.TD + a.o_begin + col] = ok ? acc : (G.nno ? __longlong_as_double(0x7ff8000000000000ll) : 0.0);
 		__syncwarp();
@@ -1773,9 +1777,7 @@ __global__ void __launch_bounds__(BLOCK, E * QH > 16 ? 2 : 3) fwd_f64_gather_ker
 			__syncwarp();
 			for (int d = lane; d < a.dim; d += 32) xs[d] = a.x[(size_t)p * a.dim + d];
 			__syncwarp();
-#pragma unroll
-			for (int e = 0; e < E; e++)
-				acc[e] = walk_column<8>(G, xs, wbase, reinterpret_cast<uint32_t*>(wbase + CLIST), lane, col + e, col + e < a.TD);
+			walk_columns<E, CDEPTH / E>(G, xs, wbase, reinterpret_cast<uint32_t*>(wbase + CLIST), lane, col, cin, acc);
 			__syncwarp();
 		}
 #pragma unroll
@@ -1973,7 +1975,7 @@ __global__ void __launch_bounds__((NC + NP) * 32) fwd_f64_stage_kernel(const __g
 				double* xs = base + CLIST + CLIST / 2;
 				for (int d = lane; d < a.dim; d += 32) xs[d] = a.x[(size_t)p * a.dim + d];
 				__syncwarp();
-				acc = walk_column<16>(G, xs, base, reinterpret_cast<uint32_t*>(base + CLIST), lane, col, col < a.TD);
+				walk_columns<1, CDEPTH>(G, xs, base, reinterpret_cast<uint32_t*>(base + CLIST), lane, col, col < a.TD, &acc);
 			}
 		}
 		if (warp < NC && col < a.TD)
@@ -3732,9 +3734,15 @@ struct ListPlan
 // 0.26 ms up to 3,000 points, against 0.23 at 1,500 and 0.34 at 3,000), then
 // its throughput, and two phases move the lists through memory.
 // Lists that would hold one entry per (point, node) within LIST_DIRECT bytes
-// do; others share a pool of four times the entries that the grids' mean
-// active counts predict for uniform points, at most LIST_SCRATCH_MAX bytes.
+// do; others share a pool of LIST_FACTOR times the entries that the grids' mean
+// active counts predict for uniform points, at least LIST_POOL_MIN, at most
+// LIST_SCRATCH_MAX bytes.  The heaviest points of d=10 to 59 grids have five to
+// thirteen times the mean, so that batches around one of them fit (four times
+// the mean did not: 300 points of 3,675 hits on a 150,000-node grid, 118
+// outputs, ran out and took 1,820 us, now 391; the one-phase kernels 820).
 constexpr size_t LIST_DIRECT = 24ull << 20;
+constexpr double LIST_FACTOR = 16.0;
+constexpr double LIST_POOL_MIN = 2.5 * 1048576.0;   // 30 MB
 constexpr size_t LIST_SCRATCH_MAX = 256ull << 20;
 constexpr double LIST_POINTS = 8192.0;
 // Phase 2 by blocks while there are at most this many (point, 32 outputs) per
@@ -3775,7 +3783,7 @@ ListPlan list_plan(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng,
 	const long long all = P.items * c;
 	P.pooled = all * 12 > (long long)LIST_DIRECT;
 	const long long most_entries = (long long)(LIST_SCRATCH_MAX - 256 - ((size_t)P.items * 8 + 255)) / 12;
-	P.cap = !P.pooled ? all : (long long)std::min({ nodes, std::max(4.0 * active, 1048576.0), (double)most_entries });
+	P.cap = !P.pooled ? all : (long long)std::min({ nodes, std::max(LIST_FACTOR * active, LIST_POOL_MIN), (double)most_entries });
 	// a pool that may not hold what is expected is not worth its walk
 	if (P.cap <= 0 || (P.pooled && active > 0.75 * (double)P.cap)) return ListPlan{};
 	P.bytes = 256 + (((size_t)P.items * 8 + 255) & ~(size_t)255) + (size_t)P.cap * 12;
@@ -4770,7 +4778,7 @@ struct HostPlan
 	unsigned long long used;
 };
 constexpr size_t HOST_PLANS_MAX = 16;
-constexpr size_t HOST_PLAN_MAX_SCRATCH = 32ull << 20;
+constexpr size_t HOST_PLAN_MAX_SCRATCH = 48ull << 20;
 // Calls whose points and values each fit this many bytes go through pinned
 // buffers that the graph itself copies from and to: one launch and one wait,
 // instead of two pageable copies around it (one point 37.1 -> 34.1 us, 16
