@@ -146,11 +146,12 @@ __device__ __forceinline__ int find_grid(const FwdArgs& a, long long p)
 }
 
 // Product of a hit node's hats in dimension order (the gold loop's `temp`).
-// Components are fetched eight at a time, so a node costs one memory round
-// trip per eight components instead of one per component.
+// Components are fetched NB at a time, so a node costs one memory round trip
+// per NB components instead of one per component: eight where 32 listed hits
+// take their weights together, four where a few lanes do.
+template <int NB = 4>
 __device__ __forceinline__ double node_weight(const GridDesc& G, const double* xs, uint32_t cptr, uint32_t ncomp)
 {
-	constexpr int NB = 8;
 	double w = 1.0;
 	for (uint32_t c0 = 0; c0 < ncomp; c0 += NB)
 	{
@@ -586,7 +587,7 @@ __global__ void __launch_bounds__(BLOCK, V * E <= 2 ? 5 : 4) fwd_f64_kernel(cons
 			const double* s64l = G.s64 + (a.o_begin + out_col<E>(0, lane) < G.ld ? a.o_begin + out_col<E>(0, lane) : 0);
 			walk_lists(G, xs, hits, lane, lo, hi, pathmask, a.chain_len[gi], [&](int m)
 			{
-				if (lane < m) hits[lane].w = node_weight(G, xs, hit_cptr(hits[lane]), hit_ncomp(hits[lane]));
+				if (lane < m) hits[lane].w = node_weight<8>(G, xs, hit_cptr(hits[lane]), hit_ncomp(hits[lane]));
 				__syncwarp();
 				int h = 0;
 				for (; h + QH <= m; h += QH)
@@ -874,13 +875,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) fwd_f32c_kernel(const __grid_cons
 // about 40 ranges.
 constexpr int SCAP = 96;
 
-// Big terms listed (16-byte entries) by the kernels of up to LISTB_MAX outputs
-// per lane: groups are taken whole at every step, so that at most a group's
-// remainder is left when a step adds up to 32.  With eight outputs per lane
-// the registers hold two FP64 rows either way, and the list only takes L1
-// from re-read rows (131,072 points, 256 outputs: 5.95 ms with it, 5.41
-// without; 118 outputs: 4.79 with, 5.31 without; 64: 1.83 and 1.98; 32: 1.54
-// and 1.77).
+// Big terms listed (16-byte entries) by the kernels with LISTB: groups are
+// taken whole at every step, so that at most a group's remainder is left when
+// a step adds up to 32.  With eight outputs per lane the registers hold two
+// FP64 rows either way, and the list only takes L1 from re-read rows (131,072
+// points, 256 outputs: 5.95 ms with it, 5.41 without), so the kernels with it
+// stop at LISTB_MAX outputs per lane; which launches take them: lists_big.
 constexpr int BCAP = 40;
 constexpr int LISTB_MAX = 4;
 
@@ -919,20 +919,20 @@ __device__ __forceinline__ uint4 pack_seg(uint32_t b, uint32_t e, double w)
 	return make_uint4(b, e, (uint32_t)__double2loint(w), (uint32_t)__double2hiint(w));
 }
 
-// QV: fine rows per group at eight outputs per lane; narrower rows take more,
-// up to FLUSH, so that a lane's loads in flight fill as many registers.
-// MINB: blocks per SM to compile for; the variant of two has room for a third
-// on rows of up to 64 outputs.
-template <int V, int E, int QV, int MINB, bool FULLROW>
-__global__ void __launch_bounds__(BLOCK, MINB == 2 && V * E <= 2 ? 3 : MINB) fwd_f32d_kernel(const __grid_constant__ FwdArgs a)
+// QV: fine rows per group; MINB: blocks per SM to compile for.  LISTB: big
+// terms are listed and read in groups, and narrow rows take more fine rows per
+// group, up to FLUSH, so that a lane's loads in flight fill as many registers
+// as QV rows of eight outputs per lane; the variant of two blocks then has
+// room for a third on rows of up to 64 outputs.
+template <int V, int E, int QV, int MINB, bool FULLROW, bool LISTB>
+__global__ void __launch_bounds__(BLOCK, LISTB && MINB == 2 && V * E <= 2 ? 3 : MINB) fwd_f32d_kernel(const __grid_constant__ FwdArgs a)
 {
-	constexpr int Q = QV * 8 / (V * E) < FLUSH ? QV * 8 / (V * E) : FLUSH;
+	constexpr int Q = !LISTB ? QV : QV * 8 / (V * E) < FLUSH ? QV * 8 / (V * E) : FLUSH;
 	// big rows per group: 32 registers of loads in flight, 64 in the variant
 	// of fewer warps (16 where that variant's third block fits beside them)
 	constexpr int QB0 = (MINB == 2 ? (V * E == 2 ? 8 : 32) : 16) / (V * E);
 	constexpr int QB = QB0 < 8 ? QB0 : 8;
-	constexpr bool LISTB = V * E <= LISTB_MAX;
-	static_assert(QB >= 2 && 31 + QB <= BCAP, "the big-term list holds a remainder and a step's hits");
+	static_assert(!LISTB || (V * E <= LISTB_MAX && QB >= 2 && 31 + QB <= BCAP), "the big-term list holds a remainder and a step's hits");
 	static_assert(FLUSH % Q == 0 || Q % FLUSH == 0, "groups of Q must tile the flush interval");
 	static_assert(32 % Q == 0, "groups of Q must tile a step's hits");
 	extern __shared__ double smem[];
@@ -1244,7 +1244,7 @@ __global__ void __launch_bounds__(BLOCK, MINB == 2 && V * E <= 2 ? 3 : MINB) fwd
 				const bool big = hit && ni.w != DESC_NONE && bound >= big_below;
 				const bool fine = hit && !big && bound >= skip_below;
 				const bool half = fine && bound < f16_below;
-				const unsigned cm = __ballot_sync(FULL, big);
+				unsigned cm = __ballot_sync(FULL, big);
 				const unsigned fm = __ballot_sync(FULL, fine && !half);
 				const unsigned hm = __ballot_sync(FULL, half);
 				const unsigned below = (1u << lane) - 1u;
@@ -1276,13 +1276,13 @@ __global__ void __launch_bounds__(BLOCK, MINB == 2 && V * E <= 2 ? 3 : MINB) fwd
 				else
 				{
 					// two at a time (two FP64 rows in flight)
-					for (unsigned c2 = cm; c2;)
+					while (cm)
 					{
-						const int k0 = __ffs(c2) - 1;
-						c2 &= c2 - 1;
-						const bool two = c2 != 0u;
-						const int k1 = two ? __ffs(c2) - 1 : k0;
-						if (two) c2 &= c2 - 1;
+						const int k0 = __ffs(cm) - 1;
+						cm &= cm - 1;
+						const bool two = cm != 0u;
+						const int k1 = two ? __ffs(cm) - 1 : k0;
+						if (two) cm &= cm - 1;
 						const double w0 = __shfl_sync(FULL, w, k0);
 						const double w1 = __shfl_sync(FULL, w, k1);
 						const double* row0 = s64l + (size_t)__shfl_sync(FULL, ni.w, k0) * ld;
@@ -1333,11 +1333,12 @@ __global__ void __launch_bounds__(BLOCK, MINB == 2 && V * E <= 2 ? 3 : MINB) fwd
 					cnt16 = rem;
 				}
 			}
-			if (cntb)
-			{
-				__syncwarp();
-				bigs(cntb);
-			}
+			if constexpr (LISTB)
+				if (cntb)
+				{
+					__syncwarp();
+					bigs(cntb);
+				}
 			if (cnt)
 			{
 				// pad to whole groups with weight-0 copies of the first entry
@@ -1611,7 +1612,7 @@ __global__ void __launch_bounds__(BLOCK, 5) walk_chunks_kernel(const __grid_cons
 					{
 						float rm = 0.f;
 						if (G.rowmax) rm = __ldg(G.rowmax + h.node);
-						w = node_weight(G, xs, hit_cptr(h), hit_ncomp(h));
+						w = node_weight<8>(G, xs, hit_cptr(h), hit_ncomp(h));
 						if (G.rowmax) keep = keeps_term(G, hit_flags(h), rm, w);
 					}
 					const unsigned km = __ballot_sync(FULL, keep);
@@ -2286,7 +2287,7 @@ __device__ __forceinline__ void point_dx(const GridDesc& G, const double* xs, do
 	walk_lists(G, xs, hits, lane, 0, G.nno, 1u, 0, [&](int m)
 	{
 		const Hit h = hits[min(lane, m - 1)];
-		const double w = lane < m ? node_weight(G, xs, hit_cptr(h), hit_ncomp(h)) : 0.0;
+		const double w = lane < m ? node_weight<8>(G, xs, hit_cptr(h), hit_ncomp(h)) : 0.0;
 		const double cs = rows_dot<R>(G.s64, (uint32_t)G.ld, h.node, m, lane, g);
 		dx_pass(G, xs, gxs + 2 * l * dim, dim, hit_cptr(h), hit_ncomp(h), cs * w, m, lane);
 		l = (l + 1) & (DXW - 1);
@@ -2458,7 +2459,7 @@ __global__ void __launch_bounds__(BLOCK) bwd_list_kernel(const __grid_constant__
 			{
 				const Hit h = hits[lane];
 				a.pair_node[at + lane] = h.node;
-				a.pair_val[at + lane] = PairVal{ node_weight(G, xs, hit_cptr(h), hit_ncomp(h)), (uint32_t)p, 0u };
+				a.pair_val[at + lane] = PairVal{ node_weight<8>(G, xs, hit_cptr(h), hit_ncomp(h)), (uint32_t)p, 0u };
 				a.pair_idx[at + lane] = (uint32_t)(at + lane);
 			}
 			at += m;
@@ -2830,25 +2831,67 @@ std::atomic<int> g_variant{[]() { const char* e = getenv("SGI_FP32C_VARIANT"); r
 // Outputs per lane of a pass of `cols` columns over rows of stride ld.
 int lane_outputs(int ld, int cols) { return ld <= 32 ? 1 : cols <= 64 ? 2 : cols <= 128 ? 4 : 8; }
 
+// FP32C kernel variants (fine rows in flight per warp against warps per SM):
+// 0 = groups of four rows, at least 3 blocks per SM; 1 = two rows, 4 blocks;
+// 2 = eight rows, 2 blocks.  With lists of big terms (lists_big), rows of up to
+// 128 outputs take more in a group, up to eight: four, eight and eight for 65
+// to 128 outputs in variants 1, 0 and 2, eight in all below, where variant 2
+// has three blocks.  They run the descent walk when every grid of the
+// launch allows it (descent_ok), else the window walk; 3-5 force the window
+// walk with the settings of 0-2.  Plans time 0-2.
+constexpr int NVARIANTS = 3;
+constexpr int NVARIANTS_ALL = 6;
+
+// A launch group's grids, by the points they get: active nodes per point,
+// expected for points uniform in the unit cube, and nodes.
+struct GroupMeans
+{
+	double active, nodes;
+};
+
+// Whether an FP32C descent launch lists its big terms.  Listing pays where
+// points have many: grids of few active nodes leave a short group per point
+// and a list to no use (us with / without it, variant 1; 131,072 points of a
+// 20,000-node d=10 grid with 39 active nodes: 32 outputs 482 / 468, 64 outputs
+// 521 / 483, 118 outputs 559 / 539; 40,000 points of a 5,000-node d=16 grid
+// with 56, 64 outputs 205 / 202; of a 40,000-node d=16 grid with 143: 64
+// outputs 318 / 327, 118 outputs 377 / 422; of a 70,000-node d=59 grid with
+// 408: 64 outputs 550 / 596, 118 outputs 739 / 820).  Variant 0 gains with
+// four outputs per lane (131,072 points on that d=59 grid: 118 outputs 1,993 /
+// 2,211), not with fewer (64 outputs 1,827 / 1,564).
+bool lists_big(int variant, bool descent, int outputs, const GroupMeans& m)
+{
+	return descent && outputs <= LISTB_MAX && variant < NVARIANTS && (variant > 0 || outputs == 4) && m.active >= 100.0;
+}
+
 // The automatic FP32C variant.  A small batch waits on its rows, with few
 // points per warp slot: more rows in flight per warp (2, then 0) beat more
-// warps (1) up to a number of points per SM that falls with the row width,
-// as a narrow row's adds hide less (d=59 and d=30 grids of 60,000 to 150,000
-// nodes; us for variants 0 / 1 / 2.  256 outputs: 10,007 points 624 / 747 /
-// 576, 20,000 990 / 1,104 / 986, 40,000 1,792 / 1,772 / 1,821.  118 outputs:
-// 4,000 264 / 327 / 246, 7,500 306 / 371 / 341, 20,000 912 / 968 / 976, 40,000
-// 1,627 / 1,568 / 1,780.  64 outputs: 4,000 230 / 235 / 214, 7,500 274 / 264 /
-// 245, 15,000 418 / 362 / 366.  32 outputs: 4,000 198 / 206 / 196, 7,500 230 /
-// 233 / 226, 15,000 339 / 314 / 336).
-// Wide rows: the line falls with the hits per point, too (15,000 points of 200
-// outputs: a 60,000-node d=45 grid of 440 active nodes 682 for 1 and 613 for
-// 2, a 40,000-node d=16 grid of 250 215 and 238).
-int auto_variant(int variant, long long npts, int sms, int outputs, double mean_active)
+// warps (1) up to a number of points per SM.  Without lists of big terms that
+// is 64 on rows of up to 128 outputs.  With them it falls with the row width,
+// as a narrow row's adds hide less (us for variants 0 / 1 / 2; a 70,000-node
+// d=59 grid with 408 active nodes and a 10,000-node d=30 grid with 126.  118
+// outputs: 1,500 points 238 / 306 / 231 and 78 / 85 / 75, 4,000 250 / 320 / 246
+// and 94 / 107 / 101, 12,000 333 / 391 / 354 and 153 / 160 / 174, 40,000 706 /
+// 739 / 875 and 354 / 356 / 436.  64 outputs, variants 1 / 2: 4,000 238 / 224
+// and 85 / 83, 12,000 284 / 277 and 127 / 129, 40,000 550 / 564 and 276 / 286.
+// 20 outputs: 4,000 216 / 197, 12,000 260 / 244, 40,000 481 / 520).  On regular
+// grids, where a point meets a fifth to a tenth of the nodes and no point far
+// more than the others, warps win earlier (118 outputs, d=10, level 4: 4,000
+// points 180 / 139 / 145, 12,000 337 / 312 / 353).
+// Above 128 outputs the line rises with the active nodes, whose longest points
+// outlast the batch (256 outputs, variants 1 / 2: 10,000 points of a
+// 100,000-node d=10 grid with 74 active nodes 116 / 131; 16,000 and 20,000 of a
+// 60,000-node d=30 grid with 321: 392 / 382 and 451 / 458; 12,000, 20,000 and
+// 40,000 of a 100,000-node d=59 grid with 501: 722 / 553, 998 / 760 and 1,267 /
+// 1,241).
+int auto_variant(int variant, long long npts, int sms, bool descent, int outputs, const GroupMeans& m)
 {
 	if (variant >= 0) return variant;
 	const long long per_sm = npts / sms;
-	if (outputs == 8) return (double)per_sm < std::min(128.0, std::max(80.0, mean_active / 4)) ? 2 : 1;
-	if (outputs == 4) return per_sm < 36 ? 2 : per_sm < 256 ? 0 : 1;
+	if (outputs == 8 && descent) return (double)per_sm < std::min(256.0, std::max(64.0, 0.35 * m.active)) ? 2 : 1;
+	if (!lists_big(1, descent, outputs, m)) return per_sm < 64 ? 2 : 1;
+	if (outputs == 4 && 16.0 * m.active > m.nodes) return per_sm < 36 ? 2 : 1;
+	if (outputs == 4) return per_sm < 18 ? 2 : per_sm < 256 ? 0 : 1;
 	return per_sm < (outputs == 2 ? 64 : 32) ? 2 : 1;
 }
 
@@ -2859,13 +2902,6 @@ uint32_t float_bits(float f)
 	return u;
 }
 
-// FP32C kernel variants (fine rows in flight per warp against warps per SM):
-// 0 = groups of four rows, at least 3 blocks per SM; 1 = two rows, 4 blocks;
-// 2 = eight rows, 2 blocks.  They run the descent walk when every grid of the
-// launch allows it (descent_ok), else the window walk; 3-5 force the window
-// walk with the settings of 0-2.  Plans time 0-2.
-constexpr int NVARIANTS = 3;
-constexpr int NVARIANTS_ALL = 6;
 template <int V, int E>
 void (*f32c_variant(int variant))(FwdArgs)
 {
@@ -2877,45 +2913,48 @@ void (*f32c_variant(int variant))(FwdArgs)
 	}
 }
 
-template <int V, int E, bool FULLROW>
+template <int V, int E, bool FULLROW, bool LISTB>
 void (*f32d_variant(int variant))(FwdArgs)
 {
 	switch (variant)
 	{
-	case 1: return fwd_f32d_kernel<V, E, 2, 4, FULLROW>;
-	case 2: return fwd_f32d_kernel<V, E, 8, 2, FULLROW>;
-	default: return fwd_f32d_kernel<V, E, 4, 3, FULLROW>;
+	case 1: return fwd_f32d_kernel<V, E, 2, 4, FULLROW, LISTB>;
+	case 2: return fwd_f32d_kernel<V, E, 8, 2, FULLROW, LISTB>;
+	default: return fwd_f32d_kernel<V, E, 4, 3, FULLROW, LISTB && V * E == 4>;   // see lists_big
 	}
 }
 
 template <int V, int E>
-void (*fp32c_kernel(int variant, bool descent, int cols))(FwdArgs)
+void (*fp32c_kernel(int variant, bool descent, int cols, bool listb))(FwdArgs)
 {
 	if (!descent || variant >= NVARIANTS) return f32c_variant<V, E>(variant);
 	// a pass whose columns fill every lane's outputs needs no column tests
-	return cols == V * 32 * E ? f32d_variant<V, E, true>(variant) : f32d_variant<V, E, false>(variant);
+	const bool full = cols == V * 32 * E;
+	if constexpr (V * E <= LISTB_MAX)
+		if (listb) return full ? f32d_variant<V, E, true, true>(variant) : f32d_variant<V, E, false, true>(variant);
+	return full ? f32d_variant<V, E, true, false>(variant) : f32d_variant<V, E, false, false>(variant);
 }
 
-void (*select_fwd(int precision, int ld, int cols, int variant = 0, bool descent = false))(FwdArgs)
+void (*select_fwd(int precision, int ld, int cols, int variant = 0, bool descent = false, bool listb = false))(FwdArgs)
 {
 	const bool f64 = precision == SGI_FP64;
-	if (ld <= 32) return f64 ? fwd_f64_kernel<1, 1> : fp32c_kernel<1, 1>(variant, descent, cols);
-	if (cols <= 64) return f64 ? fwd_f64_kernel<1, 2> : fp32c_kernel<1, 2>(variant, descent, cols);
+	if (ld <= 32) return f64 ? fwd_f64_kernel<1, 1> : fp32c_kernel<1, 1>(variant, descent, cols, listb);
+	if (cols <= 64) return f64 ? fwd_f64_kernel<1, 2> : fp32c_kernel<1, 2>(variant, descent, cols, listb);
 	// FP32C reads four consecutive outputs per lane (16-byte loads) when rows
 	// are a multiple of 128 wide
 	const bool e4 = !f64 && ld % 128 == 0;
 	if (cols <= 128)
 		return f64 ? fwd_f64_kernel<2, 2>
-		           : e4 ? fp32c_kernel<1, 4>(variant, descent, cols) : fp32c_kernel<2, 2>(variant, descent, cols);
+		           : e4 ? fp32c_kernel<1, 4>(variant, descent, cols, listb) : fp32c_kernel<2, 2>(variant, descent, cols, listb);
 	return f64 ? fwd_f64_kernel<4, 2>
-	           : e4 ? fp32c_kernel<2, 4>(variant, descent, cols) : fp32c_kernel<4, 2>(variant, descent, cols);
+	           : e4 ? fp32c_kernel<2, 4>(variant, descent, cols, false) : fp32c_kernel<4, 2>(variant, descent, cols, false);
 }
 
 // Dynamic shared memory of a forward launch.
-size_t fwd_smem(int precision, int dim, bool descent = false, int outputs = 8)
+size_t fwd_smem(int precision, int dim, bool descent = false, bool listb = false)
 {
 	if (precision != SGI_FP32C) return (size_t)WARPS * hit_stride(dim) * sizeof(double);
-	return (size_t)WARPS * (descent ? desc_stride(dim, outputs <= LISTB_MAX) : list_stride(dim)) * sizeof(double);
+	return (size_t)WARPS * (descent ? desc_stride(dim, listb) : list_stride(dim)) * sizeof(double);
 }
 
 template <int R>
@@ -3706,12 +3745,17 @@ int group_clen(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng, con
 	                 : (chunk >= maxnno ? 0 : chunk);
 }
 
-// Active nodes per point of a launch group, expected for uniform points.
-double mean_active(const sgi_grid_t* grids, int gb, int ng, const long long* pt_offsets)
+GroupMeans group_means(const sgi_grid_t* grids, int gb, int ng, const long long* pt_offsets)
 {
-	double a = 0.0;
-	for (int k = 0; k < ng; k++) a += (double)(pt_offsets[gb + k + 1] - pt_offsets[gb + k]) * grids[gb + k]->mean_active;
-	return a / (double)std::max(1ll, pt_offsets[gb + ng] - pt_offsets[gb]);
+	GroupMeans m{ 0.0, 0.0 };
+	for (int k = 0; k < ng; k++)
+	{
+		const double n = (double)(pt_offsets[gb + k + 1] - pt_offsets[gb + k]);
+		m.active += n * grids[gb + k]->mean_active;
+		m.nodes += n * grids[gb + k]->nno;
+	}
+	const double n = (double)std::max(1ll, pt_offsets[gb + ng] - pt_offsets[gb]);
+	return GroupMeans{ m.active / n, m.nodes / n };
 }
 
 // How a launch group's points run in two phases.
@@ -3979,7 +4023,7 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 		const int clen = group_clen(W, grids, gb, ng, pt_offsets, precision, chunk);
 		const int nchunks = clen ? (maxnno + clen - 1) / clen : 1;
 		const bool descent = precision == SGI_FP32C && descent_ok(grids, gb, ng, clen > 0);
-		const double active = mean_active(grids, gb, ng, pt_offsets);
+		const GroupMeans means = group_means(grids, gb, ng, pt_offsets);
 		const bool small = a.npts < (long long)W->sms * WARPS;
 		// small unchunked FP64 batches: one warp per (point, 32 outputs)
 		const bool cols_mode = precision == SGI_FP64 && small && clen == 0;
@@ -3994,10 +4038,11 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 			CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream));
 			const int cols = std::min(g0->TD - ob, PASS);
 			const int outputs = lane_outputs(g0->ld, cols);
+			const int v = auto_variant(variant, a.npts, W->sms, descent, outputs, means);
+			const bool listb = lists_big(v, descent, outputs, means);
 			const size_t smem = cols_mode ? (size_t)WARPS * cols_stride(g0->dim) * sizeof(double)
-			                              : fwd_smem(precision, g0->dim, descent, outputs);
-			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel
-				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, W->sms, outputs, active), descent);
+			                              : fwd_smem(precision, g0->dim, descent, listb);
+			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel : select_fwd(precision, g0->ld, cols, v, descent, listb);
 			if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 			int blocks = 0;
 			rc = occupancy_grid(kern, smem, W->sms, &blocks);
@@ -4486,7 +4531,7 @@ extern "C" int sgi_interpolate_noalloc(int ngrids, const sgi_grid_t* grids, cons
 		set_starts(a, grids, gb, ng);   // whole grids: the roots' groups
 		// the kernels sgi_interpolate picks for an unchunked launch
 		const bool descent = precision == SGI_FP32C && descent_ok(grids, gb, ng, false);
-		const double active = mean_active(grids, gb, ng, pt_offsets);
+		const GroupMeans means = group_means(grids, gb, ng, pt_offsets);
 		const bool small = a.npts < (long long)sms * WARPS;
 		const bool cols_mode = precision == SGI_FP64 && small;
 		for (int ob = 0; ob < g0->TD; ob += PASS)
@@ -4496,10 +4541,11 @@ extern "C" int sgi_interpolate_noalloc(int ngrids, const sgi_grid_t* grids, cons
 			CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream));
 			const int cols = std::min(g0->TD - ob, PASS);
 			const int outputs = lane_outputs(g0->ld, cols);
+			const int v = auto_variant(variant, a.npts, sms, descent, outputs, means);
+			const bool listb = lists_big(v, descent, outputs, means);
 			const size_t smem = cols_mode ? (size_t)WARPS * cols_stride(g0->dim) * sizeof(double)
-			                              : fwd_smem(precision, g0->dim, descent, outputs);
-			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel
-				: select_fwd(precision, g0->ld, cols, auto_variant(variant, a.npts, sms, outputs, active), descent);
+			                              : fwd_smem(precision, g0->dim, descent, listb);
+			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel : select_fwd(precision, g0->ld, cols, v, descent, listb);
 			if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 			int blocks = 0;
 			rc = occupancy_grid(kern, smem, sms, &blocks);

@@ -317,18 +317,24 @@ int sgi_set_chunk_rows(int rows);
 /* FP32C kernel variant used by sgi_interpolate, sgi_interpolate_host and
  * sgi_interpolate_noalloc (plans pick their own by timing among 0-2): 0 = four
  * fine surplus rows in flight per warp, 1 = two rows and more warps per SM,
- * 2 = eight rows and fewer warps.  Variants 0-2 walk the tree by descent
+ * 2 = eight rows and fewer warps.  On grids of 100 or more active nodes per
+ * point (mean over the unit cube) with rows of up to 128 outputs, variants 1
+ * and 2 (above 64 outputs, all three) also list their big terms and read more
+ * rows at once (four to eight).  Variants 0-2 walk the tree by descent
  * (child groups, see sgi_host_grid_descent) whenever every grid of a launch
  * allows it (tree depth <= 96, and <= 32 for node-chunked launches), else by
  * node windows; 3-5 are 0-2 with the node-window walk forced.  The variants
  * order the FP64 additions of big terms and of FP32 partial sums differently,
  * so their results may differ in the last bits (all within the FP32C
  * tolerance).  variant < 0 or SGI_FP32C_AUTO restores the default,
- * automatic by the points per SM and the width of a launch's rows: above 128
- * outputs 2 for fewer points per SM than a quarter of the grids' mean active
- * nodes (at least 80, at most 128), else 1; above 64 outputs 2 for fewer than
- * 36, 0 for fewer than 256, else 1; above 32 outputs 2 for fewer than 64, else
- * 1; below, 2 for fewer than 32, else 1.  Returns the previous setting
+ * automatic by the points per SM, the width of a launch's rows and its grids'
+ * mean active nodes per point, A.  Above 128 outputs: 2 for fewer points per
+ * SM than 0.35 A (at least 64, at most 256), else 1.  Up to 128 outputs with
+ * A < 100, and whenever the windows are walked: 2 for fewer than 64, else 1.
+ * Else, above 64 outputs: 2 for fewer than 18, 0 for fewer than 256, else 1
+ * (where A is more than a sixteenth of the nodes: 2 for fewer than 36, else
+ * 1); above 32 outputs 2 for fewer than 64, else 1; below, 2 for fewer than
+ * 32, else 1.  Returns the previous setting
  * (SGI_FP32C_AUTO for automatic), or a negative error code.  No reference
  * counterpart. */
 #define SGI_FP32C_AUTO 255
