@@ -3026,7 +3026,6 @@ struct sgi_grid
 	// two-phase batches: per LSTEP nodes, 32 words {length of
 	// the chunk start's ancestor chain, chain node at depth 1..length}
 	uint32_t* ctab = nullptr;
-	int nlch = 0;
 	double mean_active = 0.0;    // active nodes per point, mean over the unit cube
 	sgi_grid_info info{};
 };
@@ -3325,7 +3324,6 @@ int upload_image(GridImage& im, int device, sgi_grid_t* out)
 		if (!rc) rc = upload((void**)&d->ninfo, im.ninfo.data(), im.ninfo.size() * 4);
 	}
 	if (rc) { free_grid(d); return rc; }
-	d->nlch = im.nlch;
 	d->mean_active = im.mean_active;
 	d->skip_floor = d->skip_below = im.skip_floor;
 	d->f16_floor = im.f16_floor;
@@ -4570,7 +4568,7 @@ extern "C" int sgi_interpolate_noalloc(int ngrids, const sgi_grid_t* grids, cons
 // chunk launches) into a CUDA graph once and replays it with one
 // cudaGraphLaunch.  The chunk size is chosen by timing candidates on the
 // caller's own inputs the first time a (dim, largest nno, TotalDof,
-// precision, batch size) key is seen.
+// precision, batch size, kernels) key is seen.
 
 struct sgi_plan
 {
@@ -4592,11 +4590,30 @@ struct TuneKey
 {
 	int dim, maxnno, TD, precision;
 	long long npts;
+	int routes;   // plan_routes: grids of equal sizes may take other kernels
 	bool operator<(const TuneKey& o) const
 	{
-		return std::tie(dim, maxnno, TD, precision, npts) < std::tie(o.dim, o.maxnno, o.TD, o.precision, o.npts);
+		return std::tie(dim, maxnno, TD, precision, npts, routes) <
+			std::tie(o.dim, o.maxnno, o.TD, o.precision, o.npts, o.routes);
 	}
 };
+
+// Which kernels an unchunked call's groups take, as far as that follows from
+// the grids' active nodes: two phases (1) or one (2), lists of big terms (4)
+// or none (8).
+int plan_routes(const DeviceWork* W, int ngrids, const sgi_grid_t* grids, const long long* pt_offsets, int precision)
+{
+	int r = 0;
+	for (int gb = 0; gb < ngrids; gb += MAXG)
+	{
+		const int ng = std::min(MAXG, ngrids - gb);
+		r |= list_plan(W, grids, gb, ng, pt_offsets, precision, 0).bytes ? 1 : 2;
+		if (precision == SGI_FP32C)
+			r |= lists_big(1, descent_ok(grids, gb, ng, false), lane_outputs(grids[gb]->ld, std::min(grids[gb]->TD, PASS)),
+			               group_means(grids, gb, ng, pt_offsets)) ? 4 : 8;
+	}
+	return r;
+}
 std::mutex g_tune_mtx;
 struct TuneResult { int chunk, variant; float ms; };
 std::map<TuneKey, TuneResult> g_tune;
@@ -4666,7 +4683,8 @@ int plan_create(int ngrids, const sgi_grid_t* grids, const long long* pt_offsets
 	float tuned = 0.f;
 	int chunk = chunk_rows_req, variant = 0;
 	{
-		const TuneKey key{ grids[0]->dim, maxnno, grids[0]->TD, precision, npts };
+		const TuneKey key{ grids[0]->dim, maxnno, grids[0]->TD, precision, npts,
+		                   plan_routes(W, ngrids, grids, pt_offsets, precision) };
 		bool hit = false;
 		if (chunk < 0)
 		{
