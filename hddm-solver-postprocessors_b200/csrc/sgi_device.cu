@@ -3822,6 +3822,10 @@ ListPlan list_plan(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng,
 	P.clen = (int)c;
 	for (int k = 0; k < ng; k++)
 		P.items += (pt_offsets[gb + k + 1] - pt_offsets[gb + k]) * ((grids[gb + k]->nno + c - 1) / c);
+	// the items leave half of the scratch to the lists, whose entries are then
+	// numbered in 32 bits (8,192 points of 778,240 nodes, two thirds of them
+	// active: 50M items)
+	if ((double)P.items * 8 > (double)LIST_SCRATCH_MAX / 2) return ListPlan{};
 	const long long all = P.items * c;
 	P.pooled = all * 12 > (long long)LIST_DIRECT;
 	const long long most_entries = (long long)(LIST_SCRATCH_MAX - 256 - ((size_t)P.items * 8 + 255)) / 12;
