@@ -4067,13 +4067,14 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 
 // Launch count of a forward call with chunk size `chunk` >= 0 (as
 // launch_forward given the scratch its two-phase groups need), and that
-// scratch in *list_bytes.
+// scratch in *list_bytes; without list_bytes, of launch_forward without
+// scratch (the one-phase kernels).
 int count_launches(const DeviceWork* W, int ngrids, const sgi_grid_t* grids, const long long* pt_offsets,
 	int precision, int chunk, size_t* list_bytes)
 {
 	int n = 0;
 	const int passes = (grids[0]->TD + PASS - 1) / PASS;
-	*list_bytes = 0;
+	if (list_bytes) *list_bytes = 0;
 	for (int gb = 0; gb < ngrids; gb += MAXG)
 	{
 		const int ng = std::min(MAXG, ngrids - gb);
@@ -4081,8 +4082,8 @@ int count_launches(const DeviceWork* W, int ngrids, const sgi_grid_t* grids, con
 		int maxnno = 0;
 		for (int k = 0; k < ng; k++) maxnno = std::max(maxnno, grids[gb + k]->nno);
 		const int clen = chunk >= maxnno ? 0 : chunk;
-		const size_t lb = list_plan(W, grids, gb, ng, pt_offsets, precision, clen).bytes;
-		*list_bytes = std::max(*list_bytes, lb);
+		const size_t lb = list_bytes ? list_plan(W, grids, gb, ng, pt_offsets, precision, clen).bytes : 0;
+		if (list_bytes) *list_bytes = std::max(*list_bytes, lb);
 		n += lb ? 2 : passes * (clen ? (maxnno + clen - 1) / clen : 1);
 	}
 	return n;
@@ -4741,14 +4742,20 @@ int plan_create(int ngrids, const sgi_grid_t* grids, const long long* pt_offsets
 	p->tuned_ms = tuned;
 	size_t list_bytes = 0;
 	p->launches = count_launches(W, ngrids, grids, pt_offsets, precision, chunk, &list_bytes);
-	cudaError_t e = cudaMalloc(&p->counters, sizeof(unsigned long long) * std::max(p->launches, 1));
-	if (e != cudaSuccess) { free_plan(p); return fail(SGI_E_NOMEM, "cudaMalloc failed: %s", cudaGetErrorString(e)); }
 	if (list_bytes)
 	{
-		e = cudaMalloc(&p->scratch, list_bytes);
-		if (e != cudaSuccess) { free_plan(p); return fail(SGI_E_NOMEM, "cudaMalloc failed: %s", cudaGetErrorString(e)); }
 		p->scratch_bytes = list_bytes;
+		if (cudaMalloc(&p->scratch, list_bytes) != cudaSuccess)
+		{
+			// no room: the one-phase kernels, as in sgi_interpolate
+			cudaGetLastError();
+			p->scratch = nullptr;
+			p->scratch_bytes = 0;
+			p->launches = count_launches(W, ngrids, grids, pt_offsets, precision, chunk, nullptr);
+		}
 	}
+	cudaError_t e = cudaMalloc(&p->counters, sizeof(unsigned long long) * std::max(p->launches, 1));
+	if (e != cudaSuccess) { free_plan(p); return fail(SGI_E_NOMEM, "cudaMalloc failed: %s", cudaGetErrorString(e)); }
 	cudaStream_t cs = nullptr;
 	e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
 	if (e != cudaSuccess) { free_plan(p); return fail(SGI_E_CUDA, "cudaStreamCreate failed: %s", cudaGetErrorString(e)); }
@@ -4918,6 +4925,7 @@ int host_plan_call(DeviceWork* W, int ngrids, const sgi_grid_t* grids, const lon
 			clear_error();
 			return SGI_OK;
 		}
+		if (lb && !p->scratch) { sgi_plan_destroy(p); return SGI_OK; }   // no room now: not kept
 		std::lock_guard<std::mutex> lk(g_hp_mtx);
 		size_t n = 0;
 		auto lru = g_hp->end();

@@ -32,3 +32,28 @@ def test_more_chunks_than_the_scratch_holds(cuda):
     assert H.last_launch().kernels == 1
     some = [0, 1, 4095, 8000, 8191]
     assert np.array_equal(out[some], O.Gold(idx, sur).interpolate(X[some], nthreads=4))
+
+
+def test_plan_without_room_for_its_lists(cuda):
+    """A plan whose list scratch (256 MB here) finds no room on the device
+    records the one-phase kernels instead of failing."""
+    import torch
+    hg = H.HostGrid.regular(10, 5, 24, seed=1)
+    X = H.gen_points(10, 4000, kind=0, seed=2)
+    g, x = H.Grid(hg), torch.from_numpy(X).cuda()
+    out = torch.zeros((4000, 24), dtype=torch.float64, device="cuda")
+    plan = H.Plan(g, x, out, chunk_rows=0)
+    assert plan.launches == 2
+    two = plan.launch().clone()
+    del plan
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (160 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        plan = H.Plan(g, x, out.zero_(), chunk_rows=0)
+        assert plan.launches == 1
+        one = plan.launch().cpu().numpy()
+        del plan
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert np.array_equal(one, two.cpu().numpy())
+    assert np.array_equal(one, O.Gold(*hg.arrays()).interpolate(X, nthreads=4))
