@@ -1645,10 +1645,10 @@ __global__ void __launch_bounds__(BLOCK, 5) walk_chunks_kernel(const __grid_cons
 // Phase 2, rows through registers: one warp per (point, 32 * E outputs), QH
 // rows in flight; the next 32 list entries are loaded while 32 are added.
 // Bound by the longest point's round trips (1,500 points of up to 3,648 hits,
-// 118 outputs: 287 us with 8 rows of 64 outputs in flight, 226 with 16; 24
-// warps per SM of the one or 16 of the other).
+// 118 outputs: 287 us with 8 rows of 64 outputs in flight and 24 warps per SM,
+// 226 with 16 rows and 16 warps).
 template <int E, int QH>
-__global__ void __launch_bounds__(BLOCK, E * QH > 16 ? 2 : 3) fwd_f64_gather_kernel(const __grid_constant__ ListArgs a)
+__global__ void __launch_bounds__(BLOCK, 2) fwd_f64_gather_kernel(const __grid_constant__ ListArgs a)
 {
 	extern __shared__ double smem[];
 	const int lane = threadIdx.x & 31;
@@ -1789,40 +1789,40 @@ __global__ void __launch_bounds__(BLOCK, E * QH > 16 ? 2 : 3) fwd_f64_gather_ker
 	}
 }
 
-// Phase 2 through shared memory: one block per (point, 32 * NC outputs).  All
+// Phase 2 through shared memory: one block per (point, 32 outputs).  All
 // threads find the point's entries (a block-wide prefix sum over its items'
 // counts, then a search per hit); NP warps then copy the rows, SROWS to a
-// stage, into a ring of SRING stages (cp.async, 16 bytes each) while NC warps,
-// a lane per output, add the stage before.  A few points' time is one point's
+// stage, into a ring of SRING stages (cp.async, 16 bytes each) while one warp,
+// a lane per output, adds the stage before.  A few points' time is one point's
 // chain of adds (8 cycles each) and the round trips before it: 192 rows in
 // flight add at 24 cycles a row (16 states of 23,000 nodes, one point each:
 // 17 us, where one warp that copied 256 rows, waited and added them took 49).
 constexpr int SITEMS = 1024;               // items per round
 
 // rows, weights, nodes, the items' prefixes and entries, a word per warp
-template <int NC, int SROWS, int SRING, int SENTRIES>
-constexpr size_t stage_smem() { return (size_t)SRING * SROWS * NC * 256 + SENTRIES * 12 + SITEMS * 8 + 64; }
+template <int SROWS, int SRING, int SENTRIES>
+constexpr size_t stage_smem() { return (size_t)SRING * SROWS * 256 + SENTRIES * 12 + SITEMS * 8 + 64; }
 
-template <int NC, int NP, int SROWS, int SRING, int SENTRIES>
-__global__ void __launch_bounds__((NC + NP) * 32) fwd_f64_stage_kernel(const __grid_constant__ ListArgs a)
+template <int NP, int SROWS, int SRING, int SENTRIES>
+__global__ void __launch_bounds__((1 + NP) * 32) fwd_f64_stage_kernel(const __grid_constant__ ListArgs a)
 {
-	constexpr int SB = (NC + NP) * 32;         // threads
+	constexpr int SB = (1 + NP) * 32;          // threads
 	constexpr int IPT = (SITEMS + SB - 1) / SB; // items per thread
 	extern __shared__ double smem[];
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	double* rows = smem;
-	double* ew = rows + SRING * SROWS * NC * 32;
+	double* ew = rows + SRING * SROWS * 32;
 	uint32_t* en = reinterpret_cast<uint32_t*>(ew + SENTRIES);
 	uint32_t* ipre = en + SENTRIES;
 	uint32_t* ioff = ipre + SITEMS;
 	uint32_t* sums = ioff + SITEMS;
 	const uint32_t rows_s = (uint32_t)__cvta_generic_to_shared(rows);
-	const int ncg = (a.TD + 32 * NC - 1) / (32 * NC);
+	const int ncg = (a.TD + 31) / 32;
 	const uint32_t nitems = (uint32_t)(a.npts * ncg);
 	for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x)
 	{
 		const long long p = it / (uint32_t)ncg;
-		const int cb = (int)(it % (uint32_t)ncg) * 32 * NC, col = cb + tid;   // a consumer's output
+		const int cb = (int)(it % (uint32_t)ncg) * 32, col = cb + tid;   // an adding lane's output
 		const int gi = list_grid(a, p);
 		const GridDesc& G = a.g[gi];
 		const int nch = a.nch[gi];
@@ -1863,7 +1863,7 @@ __global__ void __launch_bounds__((NC + NP) * 32) fwd_f64_stage_kernel(const __g
 			__syncthreads();
 			uint32_t before = incl - mine, T = 0;
 #pragma unroll
-			for (int s = 0; s < NC + NP; s++)
+			for (int s = 0; s < 1 + NP; s++)
 			{
 				if (s < warp) before += sums[s];
 				T += sums[s];
@@ -1919,36 +1919,36 @@ __global__ void __launch_bounds__((NC + NP) * 32) fwd_f64_stage_kernel(const __g
 				__syncthreads();
 				const int nst = (M + SROWS - 1) / SROWS;
 				// stage st's rows, by the copying warps (a commit per stage, empty past the last)
-				const int ptid = tid - NC * 32;
-				const int ch = ptid & (NC * 16 - 1);              // this thread's 16 bytes of a row
+				const int ptid = tid - 32;
+				const int ch = ptid & 15;                         // this thread's 16 bytes of a row
 				const bool cin = cb + 2 * ch < G.ld;
 				const double* src = G.s64 + (cin ? cb + 2 * ch : 0);
-				constexpr int RSTEP = NP * 32 / (NC * 16);        // rows copied at a time
+				constexpr int RSTEP = NP * 2;                     // rows copied at a time
 				auto issue = [&](int st)
 				{
 					if (st < nst)
 					{
 						const int cnt = min(SROWS, M - st * SROWS);
 						const uint32_t* n = en + st * SROWS;
-						const uint32_t dst = rows_s + (uint32_t)(st % SRING) * (SROWS * NC * 256) + (uint32_t)ch * 16u;
+						const uint32_t dst = rows_s + (uint32_t)(st % SRING) * (SROWS * 256) + (uint32_t)ch * 16u;
 #pragma unroll 8
-						for (int r = ptid / (NC * 16); r < cnt; r += RSTEP)
+						for (int r = ptid / 16; r < cnt; r += RSTEP)
 							if (cin)
-								asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + (uint32_t)r * (NC * 256u)),
+								asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + (uint32_t)r * 256u),
 									"l"(src + (size_t)n[r] * (uint32_t)G.ld) : "memory");
 					}
 					asm volatile("cp.async.commit_group;" ::: "memory");
 				};
-				if (warp >= NC)
+				if (warp)
 					for (int st = 0; st < SRING - 1; st++) issue(st);
 				for (int st = 0; st < nst; st++)
 				{
-					if (warp >= NC) asm volatile("cp.async.wait_group %0;" :: "n"(SRING - 2) : "memory");
+					if (warp) asm volatile("cp.async.wait_group %0;" :: "n"(SRING - 2) : "memory");
 					__syncthreads();   // stage st has landed, stage st - 1 has been added
-					if (warp >= NC) issue(st + SRING - 1);
+					if (warp) issue(st + SRING - 1);
 					else
 					{
-						const double* r = rows + (size_t)(st % SRING) * (SROWS * NC * 32) + tid;
+						const double* r = rows + (size_t)(st % SRING) * (SROWS * 32) + tid;
 						const double* w = ew + st * SROWS;
 						const int cnt = min(SROWS, M - st * SROWS);
 						int q = 0;
@@ -1956,30 +1956,29 @@ __global__ void __launch_bounds__((NC + NP) * 32) fwd_f64_stage_kernel(const __g
 						{
 							double t[16];
 #pragma unroll
-							for (int j = 0; j < 16; j++) t[j] = __dmul_rn(w[q + j], r[(q + j) * (NC * 32)]);
+							for (int j = 0; j < 16; j++) t[j] = __dmul_rn(w[q + j], r[(q + j) * 32]);
 #pragma unroll
 							for (int j = 0; j < 16; j++) acc = __dadd_rn(acc, t[j]);
 						}
-						for (; q < cnt; q++) acc = __dadd_rn(acc, __dmul_rn(w[q], r[q * (NC * 32)]));
+						for (; q < cnt; q++) acc = __dadd_rn(acc, __dmul_rn(w[q], r[q * 32]));
 					}
 				}
-				if (warp >= NC) asm volatile("cp.async.wait_group 0;" ::: "memory");
+				if (warp) asm volatile("cp.async.wait_group 0;" ::: "memory");
 				__syncthreads();   // before the entries are replaced
 			}
 		}
 		if (over && !bad)
 		{
-			// items found no room: each consumer walks the point for its outputs
-			double* base = rows + (size_t)warp * cols_stride(a.dim);
-			if (warp < NC)
+			// items found no room: the adding warp walks the point for its outputs
+			if (warp == 0)
 			{
-				double* xs = base + CLIST + CLIST / 2;
+				double* xs = rows + CLIST + CLIST / 2;
 				for (int d = lane; d < a.dim; d += 32) xs[d] = a.x[(size_t)p * a.dim + d];
 				__syncwarp();
-				walk_columns<1, CDEPTH>(G, xs, base, reinterpret_cast<uint32_t*>(base + CLIST), lane, col, col < a.TD, &acc);
+				walk_columns<1, CDEPTH>(G, xs, rows, reinterpret_cast<uint32_t*>(rows + CLIST), lane, col, col < a.TD, &acc);
 			}
 		}
-		if (warp < NC && col < a.TD)
+		if (warp == 0 && col < a.TD)
 			a.out[(size_t)p * a.TD + col] = !bad ? acc : (G.nno ? __longlong_as_double(0x7ff8000000000000ll) : 0.0);
 		__syncthreads();
 	}
@@ -3900,11 +3899,11 @@ int launch_lists(const DeviceWork* W, const ListPlan& P, const sgi_grid_t* grids
 	// (point, 32 outputs) blocks for a few waves of them; beyond, warps
 	if (stage)
 	{
-		constexpr int NC = 1, NP = 3, SROWS = 64, SRING = 4, SENTRIES = 2048;
-		void (*k2)(ListArgs) = fwd_f64_stage_kernel<NC, NP, SROWS, SRING, SENTRIES>;
-		const size_t sm2 = stage_smem<NC, SROWS, SRING, SENTRIES>();
+		constexpr int NP = 3, SROWS = 64, SRING = 4, SENTRIES = 2048;
+		void (*k2)(ListArgs) = fwd_f64_stage_kernel<NP, SROWS, SRING, SENTRIES>;
+		const size_t sm2 = stage_smem<SROWS, SRING, SENTRIES>();
 		CUDA_TRY(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
-		*phase2_threads = (NC + NP) * 32;
+		*phase2_threads = (1 + NP) * 32;
 		rc = occupancy_grid(k2, sm2, W->sms, &b2, *phase2_threads);
 		if (rc) return rc;
 		b2 = (int)std::min<long long>(b2, la.npts * ncb);
