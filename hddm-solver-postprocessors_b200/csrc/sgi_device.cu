@@ -3765,15 +3765,8 @@ struct ListPlan
 	size_t bytes = 0;        // scratch; 0: the group runs the one-phase kernels
 };
 
-// A batch runs in two phases when it is not node-chunked and, on grids that
-// keep their FP64 rows, holds fewer points than the GPU does warps; FP64 also
-// up to four points per mean active node, at most LIST_POINTS.  Beyond that,
-// one warp per point wins: its time is the longest point's chain (several
-// times the mean; 1,500 to 3,000 points of a 150,000-node d=59 grid, 118
-// outputs, 0.97 ms, 6,000 points 1.18 ms, against 0.36, 0.55 and 0.88 in two
-// phases; on a 60,000-node d=30 grid of 64 outputs, half the active nodes,
-// 0.26 ms up to 3,000 points, against 0.23 at 1,500 and 0.34 at 3,000), then
-// its throughput, and two phases move the lists through memory.
+// A batch may run in two phases when it is not node-chunked, on grids that
+// keep their FP64 rows; up to how many points: two_phase_points.
 // Lists that would hold one entry per (point, node) within LIST_DIRECT bytes
 // do; others share a pool of LIST_FACTOR times the entries that the grids' mean
 // active counts predict for uniform points, at least LIST_POOL_MIN, at most
@@ -3791,8 +3784,55 @@ constexpr double LIST_POINTS = 8192.0;
 // waves of blocks take about what the warps' longest point does.
 constexpr long long STAGE_ITEMS_PER_SM = 12;
 
+// The points of a batch up to which two phases are the faster way (in the
+// forward; `active` and `nodes` per point, `outputs` per lane).
+//
+// FP64: fewer points than the GPU holds warps, and up to four per mean active
+// node, at most LIST_POINTS.  Beyond that, one warp per point wins: its time is
+// the longest point's chain (several times the mean; 1,500 to 3,000 points of a
+// 150,000-node d=59 grid, 118 outputs, 0.97 ms, 6,000 points 1.18 ms, against
+// 0.36, 0.55 and 0.88 in two phases; on a 60,000-node d=30 grid of 64 outputs,
+// half the active nodes, 0.26 ms up to 3,000 points, against 0.23 at 1,500 and
+// 0.34 at 3,000), then its throughput, and two phases move the lists through
+// memory.  Where points meet more than a sixteenth of the nodes (regular grids:
+// a tenth to a quarter, every point as many), no chain outlasts the batch, and
+// one warp per point wins from the number of warps on (us in two phases / one;
+// d=16, level 4, 969 active of 6,049: 1,184 points of 32 outputs 142 / 84, 2,700
+// 256 / 120, of 64 outputs 290 / 144, of 118 352 / 203), on rows of more than
+// 128 outputs from half a point per active node on (200 outputs, d=16, level 5,
+// 4,845 active: 1,500 points 1,402 / 2,313, 2,700 2,379 / 2,360; level 4: 1,184
+// 219 / 254, 1,500 292 / 263).
+//
+// FP32C: fewer points than the GPU holds warps while a list entry per (point,
+// node) would fit LIST_SCRATCH_MAX (in two phases the rows are added exactly,
+// so such calls keep that).  Beyond, its one-phase kernels, which walk by
+// descent and read half the bytes, win early, and the sooner the fewer of its
+// nodes a point meets, as phase 1 walks most chunks for little: from about 30
+// points per SM times the root of the share met (24 on rows of more than 64
+// outputs, 22 of more than 128), at most 4 (2.5, 5), at least 0.65 (us in two
+// phases / one; 64 outputs: 60,000-node d=10 grid, share 1/680: 400 points 66 /
+// 56, 1,100 113 / 58; 100,000 nodes, d=30, 1/184: 250 91 / 137, 400 129 / 137,
+// 1,100 193 / 146; 150,000 nodes, d=59, 1/208: 550 164 / 192, 750 218 / 216.
+// 118 outputs on the last: 200 162 / 210, 400 237 / 210, 1,100 328 / 284; d=16,
+// level 5, 1/11: 550 434 / 524.  200 outputs: 100,000 nodes, d=30: 200 134 / 197,
+// 300 189 / 170, 1,100 288 / 240).
+double two_phase_points(const DeviceWork* W, int precision, int outputs, double active, double nodes)
+{
+	const double warps = (double)W->sms * WARPS - 1.0;
+	if (precision == SGI_FP32C)
+	{
+		const double exact = std::min(warps, (double)(LIST_SCRATCH_MAX / 12) / nodes);
+		const double slope = outputs == 8 ? 22.0 : outputs == 4 ? 24.0 : 30.0, most = outputs == 8 ? 5.0 : outputs == 4 ? 2.5 : 4.0;
+		return std::max(exact, W->sms * std::min(most, std::max(0.65, slope * std::sqrt(active / nodes))));
+	}
+	const double per_active = 16.0 * active <= nodes ? 4.0 : outputs == 8 ? 0.5 : 0.0;
+	return std::max(warps, std::min(LIST_POINTS, per_active * active));
+}
+
+// `most`: points up to which the caller takes two phases, or 0 for the
+// forward's rule.
 ListPlan list_plan(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng, const long long* pt_offsets,
-	int precision, int clen, double per_active = 4.0)
+	int precision, int clen, double most = 0.0)
 {
 	ListPlan P;
 	const long long np = pt_offsets[gb + ng] - pt_offsets[gb];
@@ -3809,8 +3849,9 @@ ListPlan list_plan(const DeviceWork* W, const sgi_grid_t* grids, int gb, int ng,
 	}
 	if (maxnno == 0) return P;
 	if ((size_t)WARPS * walk_stride(grids[gb]->dim) * sizeof(double) > 220 * 1024) return P;
-	const double most = precision == SGI_FP64 ? std::min(LIST_POINTS, per_active * active / (double)np) : 0.0;
-	if (np >= (long long)W->sms * WARPS && (double)np > most) return P;
+	const int outputs = lane_outputs(grids[gb]->ld, std::min(grids[gb]->TD, PASS));
+	if (most == 0.0) most = two_phase_points(W, precision, outputs, active / (double)np, nodes / (double)np);
+	if ((double)np > most) return P;
 	// about 96 items per SM, twice the warps it holds, but chunks no shorter
 	// than the chain table's step, and with no more than 16 hits expected (an
 	// item of a long point with a few hundred outlasts the others: 1,500 points
@@ -4283,7 +4324,8 @@ int backward_lists(DeviceWork* W, sgi_grid_t g, long long npts, const double* x,
 	CUDA_TRY(cudaStreamIsCapturing(stream, &cap));
 	if (cap != cudaStreamCaptureStatusNone) return SGI_OK;
 	const long long offs[2] = { 0, npts };
-	const ListPlan P = list_plan(W, &g, 0, 1, offs, SGI_FP64, 0, DX_LIST_PER_ACTIVE);
+	const double most = std::max((double)W->sms * WARPS - 1.0, std::min(LIST_POINTS, DX_LIST_PER_ACTIVE * g->mean_active));
+	const ListPlan P = list_plan(W, &g, 0, 1, offs, SGI_FP64, 0, most);
 	const size_t smem = (size_t)bwd_stride(g->dim) * sizeof(double) + DX_ITEMS * 8 + 64;
 	if (!P.bytes || (g->nno + P.clen - 1) / P.clen > DX_ITEMS || smem > 200 * 1024) return SGI_OK;
 	cudaMemPool_t pool = nullptr;

@@ -45,15 +45,15 @@ def test_states_and_widths(cuda, counts, nodes, td, threads):
 
 
 def test_narrow_rows_through_registers(cuda):
-    """Regular grids, whose points have a thousand hits, keep the two phases
-    for a few thousand points."""
-    hosts = [H.HostGrid.regular(10, lv, 24, seed=lv) for lv in (5, 4, 5)]
-    X = H.gen_points(10, 1900, kind=0, seed=2)
-    _check([H.Grid(h) for h in hosts], X, [O.Gold(*h.arrays()) for h in hosts], [900, 100, 900], GATHERED)
+    """Grids whose points have hundreds of hits keep the two phases for a few
+    thousand points."""
+    hosts = [H.HostGrid.adaptive(45, 100_000, 24, seed=s) for s in (5, 6)]
+    X = H.gen_points(45, 1810, kind=0, seed=2)
+    _check([H.Grid(h) for h in hosts], X, [O.Gold(*h.arrays()) for h in hosts], [900, 910], GATHERED)
 
 
 @pytest.mark.parametrize("npts,wide,narrow,td,threads", [
-    (1100, 0, 3000, 64, GATHERED), (1100, 0, 3000, 118, GATHERED), (1900, 1128, 12_000, 5, GATHERED),
+    (1100, 0, 3000, 64, GATHERED), (1100, 0, 3000, 118, GATHERED), (1900, 1000, 17_000, 5, GATHERED),
     (250, 0, 15_000, 40, STAGED)])
 def test_pool_that_runs_out(cuda, npts, wide, narrow, td, threads):
     """`narrow` nodes are narrow in three of 48 dimensions, so that uniform
