@@ -2858,9 +2858,19 @@ struct GroupMeans
 // 408: 64 outputs 550 / 596, 118 outputs 739 / 820).  Variant 0 gains with
 // four outputs per lane (131,072 points on that d=59 grid: 118 outputs 1,993 /
 // 2,211), not with fewer (64 outputs 1,827 / 1,564).
-bool lists_big(int variant, bool descent, int outputs, const GroupMeans& m)
+// A batch of few points per SM waits for its longest points, whose walk the
+// list lengthens; it pays where they have many terms for the nodes that they
+// walk past, which the active nodes times the root of their share separate
+// (11 and less lose 2 to 7 percent, 23 and more gain; variant 2, 1,300 and 4,000
+// points with / without it, 64 outputs: 100,000 nodes, d=16, 234 active,
+// product 11: 207 / 199 and 211 / 203; 200,000 nodes, d=10, 136 active, 3.5: 4,000
+// 100 / 97; gains: 12,000 nodes, d=59, 186 active, 23: 15 and 11 percent; 100,000
+// nodes, d=30, 543 active, 40: 3 and 5 percent).  That is below 64 points per SM,
+// above 64 outputs below 32, where variant 0 with lists takes over.
+bool lists_big(int variant, bool descent, int outputs, const GroupMeans& m, long long per_sm)
 {
-	return descent && outputs <= LISTB_MAX && variant < NVARIANTS && (variant > 0 || outputs == 4) && m.active >= 100.0;
+	if (!descent || outputs > LISTB_MAX || variant >= NVARIANTS || (variant == 0 && outputs < 4) || m.active < 100.0) return false;
+	return per_sm >= (outputs == 4 ? 32 : 64) || m.active * std::sqrt(m.active / m.nodes) >= 16.0;
 }
 
 // The automatic FP32C variant.  A small batch waits on its rows, with few
@@ -2888,7 +2898,7 @@ int auto_variant(int variant, long long npts, int sms, bool descent, int outputs
 	if (variant >= 0) return variant;
 	const long long per_sm = npts / sms;
 	if (outputs == 8 && descent) return (double)per_sm < std::min(256.0, std::max(64.0, 0.35 * m.active)) ? 2 : 1;
-	if (!lists_big(1, descent, outputs, m)) return per_sm < 64 ? 2 : 1;
+	if (!lists_big(1, descent, outputs, m, per_sm)) return per_sm < 64 ? 2 : 1;
 	if (outputs == 4 && 16.0 * m.active > m.nodes) return per_sm < 36 ? 2 : 1;
 	if (outputs == 4) return per_sm < 18 ? 2 : per_sm < 256 ? 0 : 1;
 	return per_sm < (outputs == 2 ? 64 : 32) ? 2 : 1;
@@ -4081,7 +4091,7 @@ int launch_forward(int ngrids, const sgi_grid_t* grids, const long long* pt_offs
 			const int cols = std::min(g0->TD - ob, PASS);
 			const int outputs = lane_outputs(g0->ld, cols);
 			const int v = auto_variant(variant, a.npts, W->sms, descent, outputs, means);
-			const bool listb = lists_big(v, descent, outputs, means);
+			const bool listb = lists_big(v, descent, outputs, means, a.npts / W->sms);
 			const size_t smem = cols_mode ? (size_t)WARPS * cols_stride(g0->dim) * sizeof(double)
 			                              : fwd_smem(precision, g0->dim, descent, listb);
 			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel : select_fwd(precision, g0->ld, cols, v, descent, listb);
@@ -4586,7 +4596,7 @@ extern "C" int sgi_interpolate_noalloc(int ngrids, const sgi_grid_t* grids, cons
 			const int cols = std::min(g0->TD - ob, PASS);
 			const int outputs = lane_outputs(g0->ld, cols);
 			const int v = auto_variant(variant, a.npts, sms, descent, outputs, means);
-			const bool listb = lists_big(v, descent, outputs, means);
+			const bool listb = lists_big(v, descent, outputs, means, a.npts / sms);
 			const size_t smem = cols_mode ? (size_t)WARPS * cols_stride(g0->dim) * sizeof(double)
 			                              : fwd_smem(precision, g0->dim, descent, listb);
 			void (*kern)(FwdArgs) = cols_mode ? fwd_f64_cols_kernel : select_fwd(precision, g0->ld, cols, v, descent, listb);
@@ -4656,7 +4666,7 @@ int plan_routes(const DeviceWork* W, int ngrids, const sgi_grid_t* grids, const 
 		r |= list_plan(W, grids, gb, ng, pt_offsets, precision, 0).bytes ? 1 : 2;
 		if (precision == SGI_FP32C)
 			r |= lists_big(1, descent_ok(grids, gb, ng, false), lane_outputs(grids[gb]->ld, std::min(grids[gb]->TD, PASS)),
-			               group_means(grids, gb, ng, pt_offsets)) ? 4 : 8;
+			               group_means(grids, gb, ng, pt_offsets), (pt_offsets[gb + ng] - pt_offsets[gb]) / W->sms) ? 4 : 8;
 	}
 	return r;
 }

@@ -1,6 +1,7 @@
 """FP32C descent kernels with and without the list of big terms, which a launch
-takes by its grids' mean active nodes (100 and more list them): a grid on
-either side and both in one call, every variant, row widths around the column
+takes by its grids' mean active nodes (100 and more list them; of few points,
+where that times the root of their share of the nodes is 16 and more): a grid
+on either side and both in one call, every variant, row widths around the column
 layouts, whole grids and node chunks, surpluses whose big terms are few and
 surpluses that make every term big."""
 import numpy as np
@@ -22,9 +23,10 @@ def _mean_active(idx):
 
 
 def _hosts(td, flat):
-    for nno, lists in ((7500, True), (1500, False)):
+    for nno, lists in ((12_000, True), (1500, False)):
         idx, sur = H.HostGrid.adaptive(30, nno, td, seed=6).arrays()
-        assert (_mean_active(idx) >= 110) if lists else (_mean_active(idx) <= 90)
+        a = _mean_active(idx)
+        assert (a >= 110 and a * np.sqrt(a / nno) >= 17) if lists else (a <= 90)
         if flat:
             sur = np.sign(sur) * (0.5 + np.abs(sur) / (1 + np.abs(sur).max()))
         yield idx, sur
