@@ -1778,7 +1778,9 @@ __global__ void __launch_bounds__(BLOCK, 2) fwd_f64_gather_kernel(const __grid_c
 			__syncwarp();
 			for (int d = lane; d < a.dim; d += 32) xs[d] = a.x[(size_t)p * a.dim + d];
 			__syncwarp();
-			walk_columns<E, CDEPTH / E>(G, xs, wbase, reinterpret_cast<uint32_t*>(wbase + CLIST), lane, col, cin, acc);
+			// with 16 rows here (128 registers instead of 110) the loop above took
+			// 4 percent longer on average; as a call of its own, 8 percent
+			walk_columns<E, 8>(G, xs, wbase, reinterpret_cast<uint32_t*>(wbase + CLIST), lane, col, cin, acc);
 			__syncwarp();
 		}
 #pragma unroll
@@ -1975,7 +1977,7 @@ __global__ void __launch_bounds__((1 + NP) * 32) fwd_f64_stage_kernel(const __gr
 				double* xs = rows + CLIST + CLIST / 2;
 				for (int d = lane; d < a.dim; d += 32) xs[d] = a.x[(size_t)p * a.dim + d];
 				__syncwarp();
-				walk_columns<1, CDEPTH>(G, xs, rows, reinterpret_cast<uint32_t*>(rows + CLIST), lane, col, col < a.TD, &acc);
+				walk_columns<1, 16>(G, xs, rows, reinterpret_cast<uint32_t*>(rows + CLIST), lane, col, col < a.TD, &acc);
 			}
 		}
 		if (warp == 0 && col < a.TD)
