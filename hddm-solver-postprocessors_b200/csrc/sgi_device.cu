@@ -2482,14 +2482,15 @@ __global__ void __launch_bounds__(BLOCK) bwd_list_kernel(const __grid_constant__
 // loaded together, then the sums are split.
 //
 // A tile's length follows from the number of pairs alone (so do the bits):
-// about TILES tiles, a little more than the warps that the GPU holds (half or
-// four times as many: within 3 % on average over 399 calls), of at most
-// TILE_MAX pairs, where a tile's start-up and its parts no longer show.  With
+// about TILES tiles, just under the 3,552 warps that 148 SMs hold at three
+// blocks each (4,096, a little over them, left a second wave nearly empty: 12,000
+// points of a regular d=10 grid, 128 outputs, dL/dsurplus alone 553 us, now 461),
+// of at most TILE_MAX pairs, where a tile's start-up and its parts no longer show.  With
 // TILE_MAX pairs at every size, and one row at a time where nodes begin, both
 // gradients of 200 points of a 20,000-node d=10 grid of 118 outputs took 533
 // us, now 186, and 1,000 points of a 100,000-node d=59 grid 1,180, now 720;
 // 32,768 points of 300,000 nodes, 128 outputs, take 5.8 ms either way.
-constexpr long long TILES = 4096;
+constexpr long long TILES = 3400;
 constexpr long long TILE_MAX = 1024;
 
 long long tile_pairs(long long npairs)
