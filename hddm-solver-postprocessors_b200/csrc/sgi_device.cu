@@ -2852,28 +2852,32 @@ struct GroupMeans
 };
 
 // Whether an FP32C descent launch lists its big terms.  Listing pays where
-// points have many: grids of few active nodes leave a short group per point
-// and a list to no use (us with / without it, variant 1; 131,072 points of a
-// 20,000-node d=10 grid with 39 active nodes: 32 outputs 482 / 468, 64 outputs
-// 521 / 483, 118 outputs 559 / 539; 40,000 points of a 5,000-node d=16 grid
-// with 56, 64 outputs 205 / 202; of a 40,000-node d=16 grid with 143: 64
-// outputs 318 / 327, 118 outputs 377 / 422; of a 70,000-node d=59 grid with
-// 408: 64 outputs 550 / 596, 118 outputs 739 / 820).  Variant 0 gains with
+// points have many: few active nodes leave a short group per point and a list
+// to no use, the sooner the narrower the rows, whose adds hide less.  us with /
+// without it, the automatic variants: 131,072 points of a 20,000-node d=10 grid
+// with 39 active nodes: 32 outputs 482 / 468, 64 outputs 521 / 483, 118 outputs
+// 559 / 539; 60,000 points: of a 10,000-node d=10 grid with 46: 8 outputs 201 /
+// 199, 64 outputs 225 / 211, 118 outputs 246 / 251; of a 4,000-node d=30 grid with
+// 75: 248 / 276, 296 / 304, 389 / 413; 40,000 points of a 70,000-node d=59 grid
+// with 408: 64 outputs 550 / 596, 118 outputs 739 / 820.  Variant 0 gains with
 // four outputs per lane (131,072 points on that d=59 grid: 118 outputs 1,993 /
 // 2,211), not with fewer (64 outputs 1,827 / 1,564).
 // A batch of few points per SM waits for its longest points, whose walk the
 // list lengthens; it pays where they have many terms for the nodes that they
-// walk past, which the active nodes times the root of their share separate
-// (11 and less lose 2 to 7 percent, 23 and more gain; variant 2, 1,300 and 4,000
-// points with / without it, 64 outputs: 100,000 nodes, d=16, 234 active,
-// product 11: 207 / 199 and 211 / 203; 200,000 nodes, d=10, 136 active, 3.5: 4,000
-// 100 / 97; gains: 12,000 nodes, d=59, 186 active, 23: 15 and 11 percent; 100,000
-// nodes, d=30, 543 active, 40: 3 and 5 percent).  That is below 64 points per SM,
-// above 64 outputs below 32, where variant 0 with lists takes over.
+// walk past: a share of a 120th and more, or active nodes times the root of the
+// share of 16 and more (variant 2, 1,300 and 4,000 points of 64 outputs with /
+// without it: 100,000 nodes, d=16, 234 active, product 11: 207 / 199 and 211 /
+// 203; 200,000 nodes, d=10, 136 active, 3.5: 4,000 100 / 97; 20,000 nodes, d=16,
+// 105 active, 7.6: 57 / 58 and 76 / 75; gains: 4,000 nodes, d=30, a 53rd: 40 / 44
+// and 54 / 59; 12,000 nodes, d=59, a 64th: 15 and 11 percent; 100,000 nodes, d=30,
+// product 40: 3 and 5 percent).
 bool lists_big(int variant, bool descent, int outputs, const GroupMeans& m, long long per_sm)
 {
-	if (!descent || outputs > LISTB_MAX || variant >= NVARIANTS || (variant == 0 && outputs < 4) || m.active < 100.0) return false;
-	return per_sm >= (outputs == 4 ? 32 : 64) || m.active * std::sqrt(m.active / m.nodes) >= 16.0;
+	if (!descent || outputs > LISTB_MAX || variant >= NVARIANTS || (variant == 0 && outputs < 4)) return false;
+	const double share = m.active / m.nodes, product = m.active * std::sqrt(share);
+	if (per_sm < (outputs == 4 ? 24 : outputs == 1 && share >= 1e-3 ? 32 : 64)) return share >= 1.0 / 120 || product >= 16.0;
+	if (outputs == 2) return m.active >= 75.0 && product >= 6.0;
+	return m.active >= 45.0 || (outputs == 1 && share >= 0.05);
 }
 
 // The automatic FP32C variant.  A small batch waits on its rows, with few
@@ -2888,8 +2892,10 @@ bool lists_big(int variant, bool descent, int outputs, const GroupMeans& m, long
 // and 85 / 83, 12,000 284 / 277 and 127 / 129, 40,000 550 / 564 and 276 / 286.
 // 20 outputs: 4,000 216 / 197, 12,000 260 / 244, 40,000 481 / 520).  On regular
 // grids, where a point meets a fifth to a tenth of the nodes and no point far
-// more than the others, warps win earlier (118 outputs, d=10, level 4: 4,000
-// points 180 / 139 / 145, 12,000 337 / 312 / 353).
+// more than the others, the batch goes in even waves of the variants' warps
+// (128 outputs, d=10, level 5: 4,000 points 390 / 349 / 336, 6,500 490 / 539 for
+// 0 / 1, 9,000 543 / 540 / 549, 20,000 1,405 / 1,457 / 1,419; d=16, level 4, 118
+// outputs, 9,000 582 / 553 / 575, 60,000 3,366 / 3,399 / 3,528).
 // Above 128 outputs the line rises with the active nodes, whose longest points
 // outlast the batch (256 outputs, variants 1 / 2: 10,000 points of a
 // 100,000-node d=10 grid with 74 active nodes 116 / 131; 16,000 and 20,000 of a
@@ -2902,8 +2908,8 @@ int auto_variant(int variant, long long npts, int sms, bool descent, int outputs
 	const long long per_sm = npts / sms;
 	if (outputs == 8 && descent) return (double)per_sm < std::min(256.0, std::max(64.0, 0.35 * m.active)) ? 2 : 1;
 	if (!lists_big(1, descent, outputs, m, per_sm)) return per_sm < 64 ? 2 : 1;
-	if (outputs == 4 && 16.0 * m.active > m.nodes) return per_sm < 36 ? 2 : 1;
-	if (outputs == 4) return per_sm < 18 ? 2 : per_sm < 256 ? 0 : 1;
+	if (outputs == 4 && 16.0 * m.active > m.nodes) return per_sm < 36 ? 2 : per_sm >= 48 && per_sm < 90 ? 1 : 0;
+	if (outputs == 4) return per_sm < (m.active >= 300.0 ? 36 : 18) ? 2 : per_sm < 256 ? 0 : 1;
 	return per_sm < (outputs == 2 ? 64 : 32) ? 2 : 1;
 }
 
@@ -3809,37 +3815,38 @@ constexpr long long STAGE_ITEMS_PER_SM = 12;
 // 0.34 at 3,000), then its throughput, and two phases move the lists through
 // memory.  Where points meet more than a sixteenth of the nodes (regular grids:
 // a tenth to a quarter, every point as many), no chain outlasts the batch, and
-// one warp per point wins from the number of warps on (us in two phases / one;
-// d=16, level 4, 969 active of 6,049: 1,184 points of 32 outputs 142 / 84, 2,700
-// 256 / 120, of 64 outputs 290 / 144, of 118 352 / 203), on rows of more than
-// 128 outputs from half a point per active node on (200 outputs, d=16, level 5,
-// 4,845 active: 1,500 points 1,402 / 2,313, 2,700 2,379 / 2,360; level 4: 1,184
-// 219 / 254, 1,500 292 / 263).
+// one warp per point wins from the number of warps on, on rows of more than 64
+// outputs a little later (us in two phases / one; d=16, level 4, 969 active of
+// 6,049: 1,184 points of 32 outputs 142 / 84, 2,700 256 / 120, of 64 outputs
+// 290 / 144; of 118 outputs 1,184 150 / 165, 1,500 228 / 173; of 200 outputs
+// 219 / 254 and 292 / 263; level 5, 4,845 active: 118 outputs 629 / 827 and
+// 1,024 / 876, 200 outputs 1,500 1,402 / 2,313, 2,700 2,379 / 2,360).
 //
 // FP32C: fewer points than the GPU holds warps while a list entry per (point,
 // node) would fit LIST_SCRATCH_MAX (in two phases the rows are added exactly,
 // so such calls keep that).  Beyond, its one-phase kernels, which walk by
 // descent and read half the bytes, win early, and the sooner the fewer of its
-// nodes a point meets, as phase 1 walks most chunks for little: from about 30
-// points per SM times the root of the share met (24 on rows of more than 64
-// outputs, 22 of more than 128), at most 4 (2.5, 5), at least 0.65 (us in two
-// phases / one; 64 outputs: 60,000-node d=10 grid, share 1/680: 400 points 66 /
-// 56, 1,100 113 / 58; 100,000 nodes, d=30, 1/184: 250 91 / 137, 400 129 / 137,
-// 1,100 193 / 146; 150,000 nodes, d=59, 1/208: 550 164 / 192, 750 218 / 216.
-// 118 outputs on the last: 200 162 / 210, 400 237 / 210, 1,100 328 / 284; d=16,
-// level 5, 1/11: 550 434 / 524.  200 outputs: 100,000 nodes, d=30: 200 134 / 197,
-// 300 189 / 170, 1,100 288 / 240).
+// nodes a point meets, as phase 1 walks most chunks for little: from 1,800
+// points per SM times the share met, at least 0.65, at most 4 (2.5 on rows of
+// more than 64 outputs, 5 where the share is a sixteenth; 5.5 of more than 128; fitted to 293 such calls: 10 %
+// faster on average than either way for all, at worst 1.28 times the faster
+// one.  us in two phases / one; 64 outputs: 60,000-node d=10 grid, share 1/680,
+// 400 points 66 / 56, 1,100 113 / 58; 100,000 nodes, d=16, 1/427, 400 97 / 141;
+// d=30, 1/184, 400 129 / 137, 1,100 193 / 146; 150,000 nodes, d=59, 1/208, 550
+// 164 / 192, 1,100 277 / 238.  118 outputs on the last: 200 162 / 210, 400 237 /
+// 210; d=16, level 5, 1/11: 550 434 / 524.  200 outputs: 150,000 nodes, d=59: 250
+// 206 / 312, 750 361 / 444; d=30: 200 134 / 197, 300 189 / 170).
 double two_phase_points(const DeviceWork* W, int precision, int outputs, double active, double nodes)
 {
 	const double warps = (double)W->sms * WARPS - 1.0;
 	if (precision == SGI_FP32C)
 	{
 		const double exact = std::min(warps, (double)(LIST_SCRATCH_MAX / 12) / nodes);
-		const double slope = outputs == 8 ? 22.0 : outputs == 4 ? 24.0 : 30.0, most = outputs == 8 ? 5.0 : outputs == 4 ? 2.5 : 4.0;
-		return std::max(exact, W->sms * std::min(most, std::max(0.65, slope * std::sqrt(active / nodes))));
+		const double most = outputs == 8 ? 5.5 : outputs == 4 ? (16.0 * active > nodes ? 5.0 : 2.5) : 4.0;
+		return std::max(exact, W->sms * std::min(most, std::max(0.65, 1800.0 * active / nodes)));
 	}
-	const double per_active = 16.0 * active <= nodes ? 4.0 : outputs == 8 ? 0.5 : 0.0;
-	return std::max(warps, std::min(LIST_POINTS, per_active * active));
+	if (16.0 * active > nodes) return std::min(LIST_POINTS, warps + (outputs == 8 ? 0.3 : outputs == 4 ? 0.05 : 0.0) * active);
+	return std::max(warps, std::min(LIST_POINTS, 4.0 * active));
 }
 
 // `most`: points up to which the caller takes two phases, or 0 for the

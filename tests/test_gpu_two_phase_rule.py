@@ -26,7 +26,7 @@ def _warps():
 
 @pytest.mark.parametrize("kind,td,precision,npts,two", [
     (REGULAR, 37, H.FP64, -1, True), (REGULAR, 37, H.FP64, 0, False), (REGULAR, 64, H.FP64, 1500, False),
-    (("regular", 10, 5), 130, H.FP64, 300, False), (("regular", 16, 5), 130, H.FP64, 300, True),
+    (("regular", 10, 5), 130, H.FP64, 250, True), (("regular", 10, 5), 130, H.FP64, 350, False), (("regular", 16, 5), 130, H.FP64, 300, True),
     (REGULAR, 118, H.FP32C, -1, True), (REGULAR, 118, H.FP32C, 0, False),
     (SPARSE, 33, H.FP32C, -1, False), (SPARSE, 33, H.FP32C, 300 - 8 * 148, True),
     (("adaptive", 59, 150_000), 118, H.FP32C, 120 - 8 * 148, True),
