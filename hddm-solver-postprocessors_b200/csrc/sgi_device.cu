@@ -2052,16 +2052,18 @@ __global__ void __launch_bounds__(BLOCK) count_kernel(const __grid_constant__ Fw
 // counts, no atomics); pair numbers are stably radix-sorted by node; each
 // pair's gout row is then read once, for its node's dL/dsurplus sum and for
 // the pair's cs (the node's surplus row stays in registers); cs * w replaces w
-// in the pair; one warp per point adds its pairs' dL/dx.  The row gathers are
+// in the pair; DXW warps per point add its pairs' dL/dx.  The row gathers are
 // what bounds it, and of the two sides gout is the smaller one (33 MB against
-// 300 MB of surplus rows for 32,768 points of a 300,000-node grid of 128
-// outputs), so its rows come from the L2.  That case: 17.9 ms with surplus
-// rows gathered per point for cs (13.4 ms of it) and gout rows per node, one
-// warp per node, for the sums (6.2); now 6.4 ms, of which the rows take 2.5
-// (14 TB/s, L1 at 77 % of its peak), dL/dx 2, the sort 1.1, the two walks 1.5.
+// 300 MB of surplus rows for 32,768 points of a 300,000-node d=59 grid of 128
+// outputs), so its rows come from the L2.  That case, with 44.8M pairs, takes
+// 8.6 ms, of which the rows take 3.3 (46 GB at 14 TB/s, L1 at 77 % of its peak),
+// dL/dx 2.2, the sort 1.2, the count 0.7 and the pairs 1.2; with surplus rows
+// gathered per point for cs (13.4 ms) and gout rows per node, one warp per
+// node, for the sums (6.2), it took 22.4.
 // dL/dx alone (bwd_points_kernel): the pairs stay with their point, which
-// gathers the surplus rows of 32 hits at a time (5,001 points, 50,000 nodes,
-// 118 outputs: 1.60 ms with two rows at a time, now 0.64).
+// gathers the surplus rows of 32 hits at a time (5,001 points, 50,000 nodes, 118
+// outputs, 2.4M to 2.7M pairs: 1.54 to 1.81 ms with two rows at a time, now 0.60
+// to 0.69).
 
 // One pair of the dL/dsurplus reduction, in point order: the weight, then
 // cs * w once the node's warp has it.
@@ -2489,7 +2491,7 @@ __global__ void __launch_bounds__(BLOCK) bwd_list_kernel(const __grid_constant__
 // TILE_MAX pairs at every size, and one row at a time where nodes begin, both
 // gradients of 200 points of a 20,000-node d=10 grid of 118 outputs took 533
 // us, now 186, and 1,000 points of a 100,000-node d=59 grid 1,180, now 720;
-// 32,768 points of 300,000 nodes, 128 outputs, take 5.8 ms either way.
+// 44.8M pairs of 128 outputs take 8.6 ms either way.
 constexpr long long TILES = 3400;
 constexpr long long TILE_MAX = 1024;
 

@@ -317,10 +317,12 @@ int sgi_set_chunk_rows(int rows);
 /* FP32C kernel variant used by sgi_interpolate, sgi_interpolate_host and
  * sgi_interpolate_noalloc (plans pick their own by timing among 0-2): 0 = four
  * fine surplus rows in flight per warp, 1 = two rows and more warps per SM,
- * 2 = eight rows and fewer warps.  On grids of 100 or more active nodes per
- * point (mean over the unit cube) with rows of up to 128 outputs, variants 1
- * and 2 (above 64 outputs, all three) also list their big terms and read more
- * rows at once (four to eight).  Variants 0-2 walk the tree by descent
+ * 2 = eight rows and fewer warps.  On rows of up to 128 outputs, where points
+ * meet many nodes (about 45 active nodes per point, mean over the unit cube; 75
+ * on rows of 33 to 64 outputs; in small batches a 120th of the nodes, or 16 as
+ * active nodes times the root of their share), variants 1 and 2 (above 64
+ * outputs, all three) also list their big terms and read more rows at once
+ * (four to eight).  Variants 0-2 walk the tree by descent
  * (child groups, see sgi_host_grid_descent) whenever every grid of a launch
  * allows it (tree depth <= 96, and <= 32 for node-chunked launches), else by
  * node windows; 3-5 are 0-2 with the node-window walk forced.  The variants
@@ -329,12 +331,12 @@ int sgi_set_chunk_rows(int rows);
  * tolerance).  variant < 0 or SGI_FP32C_AUTO restores the default,
  * automatic by the points per SM, the width of a launch's rows and its grids'
  * mean active nodes per point, A.  Above 128 outputs: 2 for fewer points per
- * SM than 0.35 A (at least 64, at most 256), else 1.  Up to 128 outputs with
- * A < 100, and whenever the windows are walked: 2 for fewer than 64, else 1.
- * Else, above 64 outputs: 2 for fewer than 18, 0 for fewer than 256, else 1
- * (where A is more than a sixteenth of the nodes: 2 for fewer than 36, else
- * 1); above 32 outputs 2 for fewer than 64, else 1; below, 2 for fewer than
- * 32, else 1.  Returns the previous setting
+ * SM than 0.35 A (at least 64, at most 256), else 1.  Without lists, and
+ * whenever the windows are walked: 2 for fewer than 64, else 1.  With lists,
+ * above 64 outputs: 2 for fewer than 18 (36 from A = 300 on), 0 for fewer than
+ * 256, else 1 (where A is more than a sixteenth of the nodes: 2 for fewer than
+ * 36, 1 for 48 to 89, else 0); above 32 outputs 2 for fewer than 64, else 1;
+ * below, 2 for fewer than 32, else 1.  Returns the previous setting
  * (SGI_FP32C_AUTO for automatic), or a negative error code.  No reference
  * counterpart. */
 #define SGI_FP32C_AUTO 255
@@ -343,9 +345,9 @@ int sgi_set_fp32c_variant(int variant);
 /* Plans: one forward call recorded into a CUDA graph and replayed.
  * sgi_plan_create records every launch of sgi_interpolate(ngrids, grids,
  * pt_offsets, x, out, precision) (work-counter clears and node-chunk launches,
- * with work counters, and the hit lists of small batches, owned by the plan)
- * into a graph; sgi_plan_launch replays
- * it on `stream` with one cudaGraphLaunch.  x and out are baked into the
+ * with work counters, and the hit lists of small batches, at most 256 MB, owned
+ * by the plan; without room for the lists, the kernels that need none) into a
+ * graph; sgi_plan_launch replays it on `stream` with one cudaGraphLaunch.  x and out are baked into the
  * graph: later replays read the same x buffer and write the same out buffer.
  * chunk_rows >= 0 fixes the node-chunk size (0 = none); chunk_rows < 0 lets the
  * autotuner choose it: the first time a (dim, largest nno, TotalDof,
